@@ -326,24 +326,14 @@ int flare_kv_alloc(flare_attn_ctx* ctx, int num_layers, int batch, int max_seq_l
             return code;
         }
     }
-    if (kv_dtype == FLARE_KV_Q8_0 && (head_dim == 64 || head_dim == 128) && num_kv_heads <= 8) {
-        CUtensorMapSwizzle swz = head_dim == 64 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B;
-        // preferred: (head_dim bytes, slot, kv head, layer*batch + seq) with a box of 32 slots x all heads,
-        // which lands in shared memory as [head][slot][head_dim] from one contiguous stretch of the plane
-        const uint64_t dims_w[4] = {(uint64_t)head_dim, (uint64_t)max_seq_len, (uint64_t)num_kv_heads, (uint64_t)num_layers * batch};
-        const uint64_t strides_w[3] = {(uint64_t)kvd, (uint64_t)head_dim, (uint64_t)max_seq_len * kvd};
-        const uint32_t box_w[4] = {(uint32_t)head_dim, 32, (uint32_t)num_kv_heads, 1};
-        int r1 = flare_make_tensor_map(&kv->kq_map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 4, kv->plane[FLARE_PLANE_K_Q], dims_w, strides_w, box_w, swz);
-        int r2 = flare_make_tensor_map(&kv->vq_map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 4, kv->plane[FLARE_PLANE_V_Q], dims_w, strides_w, box_w, swz);
-        kv->maps_whole_rows = (r1 == 0 && r2 == 0);
-        if (!kv->maps_whole_rows) {
-            // fallback: natural dimension order, one box per head
-            const uint64_t dims[4] = {(uint64_t)head_dim, (uint64_t)num_kv_heads, (uint64_t)max_seq_len, (uint64_t)num_layers * batch};
-            const uint64_t strides[3] = {(uint64_t)head_dim, (uint64_t)kvd, (uint64_t)max_seq_len * kvd};
-            const uint32_t box[4] = {(uint32_t)head_dim, 1, 32, 1};
-            r1 = flare_make_tensor_map(&kv->kq_map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 4, kv->plane[FLARE_PLANE_K_Q], dims, strides, box, swz);
-            r2 = flare_make_tensor_map(&kv->vq_map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 4, kv->plane[FLARE_PLANE_V_Q], dims, strides, box, swz);
-        }
+    if (kv_dtype == FLARE_KV_Q8_0 && (head_dim == 64 || head_dim == 128) && num_kv_heads <= 8 && kvd % 128 == 0) {
+        // (128 bytes of heads, slot, group of heads, layer*batch + seq) with a box of 32 slots x all heads, which lands in
+        // shared memory as [group][slot][128] from one contiguous stretch of the plane
+        const uint64_t dims_w[4] = {128, (uint64_t)max_seq_len, (uint64_t)kvd / 128, (uint64_t)num_layers * batch};
+        const uint64_t strides_w[3] = {(uint64_t)kvd, 128, (uint64_t)max_seq_len * kvd};
+        const uint32_t box_w[4] = {128, 32, (uint32_t)(kvd / 128), 1};
+        int r1 = flare_make_tensor_map(&kv->kq_map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 4, kv->plane[FLARE_PLANE_K_Q], dims_w, strides_w, box_w, CU_TENSOR_MAP_SWIZZLE_128B);
+        int r2 = flare_make_tensor_map(&kv->vq_map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 4, kv->plane[FLARE_PLANE_V_Q], dims_w, strides_w, box_w, CU_TENSOR_MAP_SWIZZLE_128B);
         if (r1 != 0 || r2 != 0) {
             flare_set_error(ctx, FLARE_ERR_CUDA, "cuTensorMapEncodeTiled failed (%d, %d)", r1, r2);
             flare_kv_free(kv);
@@ -454,16 +444,22 @@ int flare_kv_append_f32(flare_kv* kv, int layer, int seq, int n_rows, const floa
     return FLARE_OK;
 }
 
-static int upload_small(flare_attn_ctx* ctx, const flare_kv* kv, int n_q, const int* attend_len, const int** d_attend,
-                        const int2** d_ring, int* max_attend);
+static int small_arrays(flare_attn_ctx* ctx, const flare_kv* kv, int n_q, const int* attend_len, int* max_attend);
+static int upload_small(flare_attn_ctx* ctx, int B, const int** d_attend, const int2** d_ring);
+// The ring positions of a decode step on the device.
+static int step_ring(flare_kv* kv, const int2** d_ring) {
+    const int* d_att; int mx;
+    FLARE_TRY(small_arrays(kv->ctx, kv, 1, nullptr, &mx));
+    return upload_small(kv->ctx, kv->batch, &d_att, d_ring);
+}
 
 int flare_kv_write_step_f32(flare_kv* kv, int layer, const float* key, const float* value, int on_device) {
     FLARE_TRY(check_layer_seq(kv, layer, 0));
     flare_attn_ctx* ctx = kv->ctx;
     if (!key || !value) return flare_set_error(ctx, FLARE_ERR_INVALID_ARG, "flare_kv_write_step_f32: null rows");
     BIND(ctx);
-    const int* d_att; const int2* d_ring; int mx;
-    FLARE_TRY(upload_small(ctx, kv, 1, nullptr, &d_att, &d_ring, &mx));
+    const int2* d_ring;
+    FLARE_TRY(step_ring(kv, &d_ring));
     const float *dk, *dv;
     bool must_sync;
     FLARE_TRY(stage_rows(ctx, key, value, (size_t)kv->batch * kv->kv_dim, on_device, &dk, &dv, &must_sync));
@@ -516,8 +512,8 @@ int flare_kv_write_step_rope_f32(flare_kv* kv, int layer, const float* key, cons
     BIND(ctx);
     const long long* d_pos = nullptr;
     FLARE_TRY(upload_positions(kv, positions, kv->batch, &d_pos));
-    const int* d_att; const int2* d_ring; int mx;
-    FLARE_TRY(upload_small(ctx, kv, 1, nullptr, &d_att, &d_ring, &mx));
+    const int2* d_ring;
+    FLARE_TRY(step_ring(kv, &d_ring));
     const float *dk, *dv;
     bool must_sync;
     FLARE_TRY(stage_rows(ctx, key, value, (size_t)kv->batch * kv->kv_dim, on_device, &dk, &dv, &must_sync));
@@ -542,8 +538,8 @@ int flare_kv_write_step_rope_device(flare_kv* kv, int layer, const float* d_key,
     FLARE_TRY(check_layer_seq(kv, layer, 0));
     flare_attn_ctx* ctx = kv->ctx;
     BIND(ctx);
-    const int* d_att; const int2* d_ring; int mx;
-    FLARE_TRY(upload_small(ctx, kv, 1, nullptr, &d_att, &d_ring, &mx));
+    const int2* d_ring;
+    FLARE_TRY(step_ring(kv, &d_ring));
     if (kv->dtype == FLARE_KV_KIVI_REF || kv->dtype == FLARE_KV_KIVI_G32) {
         const size_t bytes = (size_t)kv->batch * kv->kv_dim * sizeof(float);
         FLARE_TRY(flare_ensure(ctx, &ctx->d_conv, &ctx->conv_bytes, bytes));
@@ -713,19 +709,12 @@ int flare_kv_export_dequant(flare_kv* kv, int layer, int seq, float* k_out, floa
 }
 
 // ---------------------------------------------------------------- attention
-// Small per-call integer arrays (attend_len, ring state) go through pinned memory.
-static int upload_small(flare_attn_ctx* ctx, const flare_kv* kv, int n_q, const int* attend_len, const int** d_attend,
-                        const int2** d_ring, int* max_attend) {
+// The per-sequence attend lengths and ring states of a call, on the host: [ring (position, length)][attend].
+static int small_arrays(flare_attn_ctx* ctx, const flare_kv* kv, int n_q, const int* attend_len, int* max_attend) {
     const int B = kv->batch;
-    size_t bytes = (size_t)B * (sizeof(int) + sizeof(int2));
-    // a ring of pinned/device slots so that back-to-back calls do not overwrite in-flight data
-    const int kSlots = FLARE_SMALL_SLOTS;
-    size_t slot_bytes = (bytes + 255) / 256 * 256;
-    // build the arrays first; a decode step makes one call per layer with identical contents,
-    // in which case the device copy of the previous call is reused and nothing is uploaded
-    std::vector<int> cur((size_t)B * 3);
-    int2* c_ring = (int2*)cur.data();
-    int* c_att = cur.data() + 2 * (size_t)B;
+    ctx->small_cur.resize((size_t)B * 3);
+    int2* c_ring = (int2*)ctx->small_cur.data();
+    int* c_att = ctx->small_cur.data() + 2 * (size_t)B;
     int mx = 0;
     for (int b = 0; b < B; b++) {
         int64_t a;
@@ -738,37 +727,54 @@ static int upload_small(flare_attn_ctx* ctx, const flare_kv* kv, int n_q, const 
         c_ring[b] = make_int2((int)kv->position[b], (int)kv->length[b]);
     }
     *max_attend = mx;
-    if (ctx->small_last_dev && cur == ctx->small_last) {
-        *d_ring = (const int2*)ctx->small_last_dev;
-        *d_attend = (const int*)((const char*)ctx->small_last_dev + (size_t)B * sizeof(int2));
-        return FLARE_OK;
+    return FLARE_OK;
+}
+// The same on the device, through a ring of page-locked slots so that back-to-back calls do not overwrite data in
+// flight.  A decode step makes one call per layer with identical contents, in which case the device copy of the
+// previous call is reused and nothing is uploaded.
+static int upload_small(flare_attn_ctx* ctx, int B, const int** d_attend, const int2** d_ring) {
+    const size_t bytes = (size_t)B * (sizeof(int) + sizeof(int2));
+    const int kSlots = FLARE_SMALL_SLOTS;
+    const size_t slot_bytes = (bytes + 255) / 256 * 256;
+    if (!ctx->small_last_dev || ctx->small_cur != ctx->small_last) {
+        if (slot_bytes * kSlots > ctx->pinned_bytes || slot_bytes * kSlots > ctx->misc_bytes) {
+            FLARE_TRY(flare_ensure_pinned(ctx, slot_bytes * kSlots));
+            FLARE_TRY(flare_ensure(ctx, &ctx->d_misc, &ctx->misc_bytes, slot_bytes * kSlots));
+        }
+        const int slot = (int)(ctx->small_counter++ % kSlots);
+        const size_t off = (size_t)slot * slot_bytes;
+        if (!ctx->small_events[slot]) FLARE_CUDA_OK(ctx, cudaEventCreateWithFlags(&ctx->small_events[slot], cudaEventDisableTiming));
+        else FLARE_CUDA_OK(ctx, cudaEventSynchronize(ctx->small_events[slot]));   // the copy that last used this slot is done
+        memcpy((char*)ctx->h_pinned + off, ctx->small_cur.data(), bytes);
+        char* d = (char*)ctx->d_misc + off;
+        FLARE_CUDA_OK(ctx, cudaMemcpyAsync(d, (char*)ctx->h_pinned + off, bytes, cudaMemcpyHostToDevice, ctx->stream));
+        FLARE_CUDA_OK(ctx, cudaEventRecord(ctx->small_events[slot], ctx->stream));
+        ctx->small_last = ctx->small_cur;
+        ctx->small_last_dev = d;
     }
-    if (slot_bytes * kSlots > ctx->pinned_bytes || slot_bytes * kSlots > ctx->misc_bytes) {
-        FLARE_TRY(flare_ensure_pinned(ctx, slot_bytes * kSlots));
-        FLARE_TRY(flare_ensure(ctx, &ctx->d_misc, &ctx->misc_bytes, slot_bytes * kSlots));
-    }
-    const int slot = (int)(ctx->small_counter++ % kSlots);
-    size_t off = (size_t)slot * slot_bytes;
-    if (!ctx->small_events[slot]) FLARE_CUDA_OK(ctx, cudaEventCreateWithFlags(&ctx->small_events[slot], cudaEventDisableTiming));
-    else FLARE_CUDA_OK(ctx, cudaEventSynchronize(ctx->small_events[slot]));   // the copy that last used this slot is done
-    memcpy((char*)ctx->h_pinned + off, cur.data(), bytes);
-    char* d = (char*)ctx->d_misc + off;
-    FLARE_CUDA_OK(ctx, cudaMemcpyAsync(d, (char*)ctx->h_pinned + off, bytes, cudaMemcpyHostToDevice, ctx->stream));
-    FLARE_CUDA_OK(ctx, cudaEventRecord(ctx->small_events[slot], ctx->stream));
-    *d_ring = (const int2*)d;
-    *d_attend = (const int*)(d + (size_t)B * sizeof(int2));
-    ctx->small_last.swap(cur);
-    ctx->small_last_dev = d;
-    *max_attend = mx;
+    *d_ring = (const int2*)ctx->small_last_dev;
+    *d_attend = (const int*)((const char*)ctx->small_last_dev + (size_t)B * sizeof(int2));
     return FLARE_OK;
 }
 
+}  // extern "C"
+
+int flare_small_on_device(flare_attn_ctx* ctx, const DecodeArgs& a, const int** d_attend, const int2** d_ring) {
+    if (a.attend_len) { *d_attend = a.attend_len; *d_ring = a.ring; return FLARE_OK; }
+    return upload_small(ctx, a.batch, d_attend, d_ring);
+}
+
+extern "C" {
+
+// fuse, when non-null: the new rows this single-query call stores first (and the rotation, the output form): done by the
+// attention kernel where it can, by kernels of their own in front of it otherwise.
 // q_staged: when non-null, q is already on the device there although `out` is a host buffer (on_device = 0).
 // multi: the slot range is this rank's share of one sequence; the records of all ranks are exchanged and merged
 // (flare_multi_tail) and `out` receives the attention output over the whole sequence.
 int flare_decode_common(flare_attn_ctx* ctx, flare_kv* kv, int layer, int num_heads, const float* q, int n_q,
                         const int* attend_len, float softcap, int slot_begin, int slot_end, int want_partial,
-                        int causal_q, float* out, int on_device, const float* q_staged, int multi) {
+                        int causal_q, float* out, int on_device, const float* q_staged, int multi, const StepFusion* fuse,
+                        size_t q_seq_stride) {
     CHECK_CTX(ctx);
     if (!kv || kv->ctx != ctx) return flare_set_error(ctx, FLARE_ERR_STATE, "no KV cache bound to this context");
     if (layer < 0 || layer >= kv->num_layers) return flare_set_error(ctx, FLARE_ERR_INVALID_ARG, "layer %d out of range", layer);
@@ -786,12 +792,13 @@ int flare_decode_common(flare_attn_ctx* ctx, flare_kv* kv, int layer, int num_he
     a.window = 0;
     a.kmap = kv->has_maps ? &kv->kq_map : nullptr;
     a.vmap = kv->has_maps ? &kv->vq_map : nullptr;
-    a.whole_rows = kv->maps_whole_rows ? 1 : 0;
     a.kv_obj = kv;
     a.batch = kv->batch; a.n_q = n_q; a.num_heads = num_heads;
     a.slot_begin = slot_begin; a.slot_end = slot_end; a.want_partial = want_partial; a.causal_q = causal_q;
-    FLARE_TRY(upload_small(ctx, kv, n_q, attend_len, &a.attend_len, &a.ring, &a.max_attend));
-    a.h_attend = ctx->small_last.size() == (size_t)kv->batch * 3 ? ctx->small_last.data() + 2 * (size_t)kv->batch : nullptr;
+    FLARE_TRY(small_arrays(ctx, kv, n_q, attend_len, &a.max_attend));
+    a.h_ring = (const int2*)ctx->small_cur.data();
+    a.h_attend = ctx->small_cur.data() + 2 * (size_t)kv->batch;
+    a.q_seq_stride = q_seq_stride;
     const size_t rows = (size_t)kv->batch * n_q * num_heads;
     const size_t q_bytes = rows * kv->head_dim * 4;
     const size_t o_bytes = rows * (kv->head_dim + ((want_partial && !multi) ? 2 : 0)) * 4;
@@ -824,11 +831,18 @@ int flare_decode_common(flare_attn_ctx* ctx, flare_kv* kv, int layer, int num_he
         }
     }
     FLARE_TRY(stats_begin(ctx));
+    if (fuse && flare_decode_q8_supported(a)) a.fuse = fuse;
+    else if (fuse) {
+        const int* d_att; const int2* d_ring;
+        FLARE_TRY(flare_small_on_device(ctx, a, &d_att, &d_ring));
+        FLARE_TRY(flare_launch_kv_write_step(kv, layer, d_ring, fuse->k, fuse->v));
+        if (fuse->quantised) *fuse->quantised = false;
+    }
     FLARE_TRY(flare_launch_decode(ctx, a));
     if (multi) FLARE_TRY(flare_multi_tail(ctx, work, n_split, (int)rows, kv->head_dim, a.out));
     if (ctx->stats_on) {
         double bytes = 0.0, pairs = 0.0;
-        for (int b = 0; b < kv->batch && a.h_attend; b++) {
+        for (int b = 0; b < kv->batch; b++) {
             for (int i = 0; i < n_q; i++) {
                 int lo = 0, hi = a.h_attend[b] - (causal_q ? (n_q - 1 - i) : 0);
                 if (slot_end >= 0) { lo = slot_begin; if (hi > slot_end) hi = slot_end; }
@@ -861,11 +875,11 @@ int flare_decode_step(flare_attn_ctx* ctx, flare_kv* kv, int layer, int num_head
     if (num_heads < 1 || num_heads % kv->num_kv_heads)
         return flare_set_error(ctx, FLARE_ERR_INVALID_ARG, "num_heads %d is not a multiple of %d kv heads", num_heads, kv->num_kv_heads);
     BIND(ctx);
-    const int* d_att; const int2* d_ring; int mx;
-    FLARE_TRY(upload_small(ctx, kv, 1, nullptr, &d_att, &d_ring, &mx));
+    StepFusion f;
+    f.row_stride = kv->kv_dim;
     if (on_device) {
-        FLARE_TRY(flare_launch_kv_write_step(kv, layer, d_ring, key, value));
-        return flare_decode_common(ctx, kv, layer, num_heads, q, 1, nullptr, 0.0f, 0, -1, 0, 1, out, 1);
+        f.k = key; f.v = value;
+        return flare_decode_common(ctx, kv, layer, num_heads, q, 1, nullptr, 0.0f, 0, -1, 0, 1, out, 1, nullptr, 0, &f);
     }
     const size_t row_fl = (size_t)kv->batch * kv->kv_dim, q_fl = (size_t)kv->batch * num_heads * kv->head_dim;
     const size_t bytes = (2 * row_fl + q_fl) * sizeof(float);
@@ -906,9 +920,9 @@ int flare_decode_step(flare_attn_ctx* ctx, flare_kv* kv, int layer, int num_head
         FLARE_CUDA_OK(ctx, cudaMemcpyAsync(d + 2 * row_fl, q, q_fl * 4, cudaMemcpyHostToDevice, ctx->stream));
     }
     ctx->last_launch_overlappable = false;
-    FLARE_TRY(flare_launch_kv_write_step(kv, layer, d_ring, dk, dv));
+    f.k = dk; f.v = dv;
     // attention on the staged q; the output goes to the caller's host buffer; one synchronisation at the end
-    return flare_decode_common(ctx, kv, layer, num_heads, q, 1, nullptr, 0.0f, 0, -1, 0, 1, out, 0, dq);
+    return flare_decode_common(ctx, kv, layer, num_heads, q, 1, nullptr, 0.0f, 0, -1, 0, 1, out, 0, dq, 0, &f);
 }
 
 int flare_decode_attn_noalloc(flare_attn_ctx* ctx, flare_kv* kv, int layer, int num_heads, const float* q_dev, int n_q,

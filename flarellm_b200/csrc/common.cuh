@@ -50,13 +50,17 @@ struct flare_attn_ctx {
     struct { const void* p; bool locked; } lock_cache[64] = {};
     unsigned lock_cache_next = 0;
     uint64_t small_counter = 0;
-    std::vector<int> small_last;       // host copy of the last uploaded (ring, attend) arrays
+    std::vector<int> small_cur;        // this call's (ring, attend) arrays, on the host
+    std::vector<int> small_last;       // host copy of the last uploaded ones
     const void* small_last_dev = nullptr;
     cudaEvent_t small_events[FLARE_SMALL_SLOTS] = {};
     int work_phase = 0;              // which half of d_work the last split-KV launch used
     // true while the last kernel put on the stream is one that never writes a cache or q, so that the
     // next decode kernel may overlap its prologue with it (programmatic dependent launch)
     bool last_launch_overlappable = false;
+    // the cache layer whose rows the last kernel on the stream stores itself (a fused step), else null: the next decode
+    // kernel may not request tiles of that layer before the stream has reached it
+    const void* last_written_layer = nullptr;
     int* h_err = nullptr;            // status word in page-locked, device-mapped host memory: a kernel whose bounded wait gives up stores a code here
     int* d_err = nullptr;            // the device's address of the same word (what kernels are given)
     int* d_gaveup = nullptr;         // device memory: set by an exchange whose wait ran out, so that the calls queued behind
@@ -82,10 +86,9 @@ struct flare_kv {
     void* plane[FLARE_PLANE_COUNT] = {};
     size_t plane_bytes[FLARE_PLANE_COUNT] = {};   // per (layer, sequence)
     std::vector<int64_t> position, length;       // per sequence
-    // TMA maps of the Q8_0 payload planes: (head_dim bytes, kv head, slot, layer*batch + seq), box 32 slots of one head
+    // TMA maps of the Q8_0 payload planes: (128 bytes = one or two heads, slot, group of heads, layer*batch + seq), box 32 slots of all heads
     CUtensorMap kq_map, vq_map;
     bool has_maps = false;
-    bool maps_whole_rows = false;
     // TMA maps of the group-32 KIVI code planes: (16 bytes = 64 codes of one head, slot, kv head, layer*batch + seq)
     CUtensorMap g32_kmap, g32_vmap;
     bool has_g32_maps = false;
@@ -117,7 +120,8 @@ int flare_set_error(flare_attn_ctx* ctx, int code, const char* fmt, ...);
 #define FLARE_LAUNCH_CHECK(ctx)                                                            \
     do {                                                                                   \
         (ctx)->launches++;                                                                 \
-        (ctx)->last_launch_overlappable = false;                                                                 \
+        (ctx)->last_launch_overlappable = false;                                           \
+        (ctx)->last_written_layer = nullptr;                                               \
         cudaError_t _e = cudaGetLastError();                                               \
         if (_e != cudaSuccess)                                                             \
             return flare_set_error((ctx), FLARE_ERR_CUDA, "kernel launch failed: %s (%s:%d)", \
@@ -136,12 +140,26 @@ struct KvLayerView {
 KvLayerView flare_layer_view(const flare_kv* kv, int layer);
 
 // ---- kernels-in-other-files entry points (host launchers) ----------------------------------
+// What a single-query decode launch does besides attending, when its kernel can (Q8_0 tensor-core path).
+struct StepFusion {
+    // the new row of every sequence, stored (and quantised) at its ring position before it is attended
+    const float *k = nullptr, *v = nullptr;
+    size_t row_stride = 0;                       // floats between the rows of two sequences
+    // rotary table and row positions (device): k and q are rotated on their way in
+    const float *cos = nullptr, *sin = nullptr;
+    const long long* positions = nullptr;
+    // output as Q8_0 input blocks (quantize_input_q8_0) instead of f32; *quantised reports whether that was done
+    int8_t* oq = nullptr;
+    float* os = nullptr;
+    bool* quantised = nullptr;
+};
 struct DecodeArgs {
     KvLayerView kv;
     const float* q;        // device [batch][n_q][nh][hd]
+    size_t q_seq_stride = 0;   // floats between the queries of two sequences (0: dense)
     float* out;            // device: final [batch][n_q][nh][hd] or partial [..][hd+2]
-    const int* attend_len; // device [batch]  (slots seen by the last query)
-    const int2* ring;      // device [batch]  (position, length) — KIVI caches need it
+    const int* attend_len = nullptr; // device [batch]  (slots seen by the last query); null: flare_small_on_device uploads h_attend
+    const int2* ring = nullptr;      // device [batch]  (position, length) — KIVI caches need it
     int batch, n_q, num_heads;
     int slot_begin, slot_end;  // restrict to [slot_begin, slot_end) (slot_end < 0: no restriction)
     int want_partial;          // 1: write [m, l, o] unnormalised
@@ -150,9 +168,10 @@ struct DecodeArgs {
     int window;                // > 0: every query reads at most its newest `window` slots (sliding-window prefill)
     int layer;
     const CUtensorMap *kmap, *vmap;   // Q8_0 payload maps (null when the cache has none)
-    int whole_rows;                   // maps deliver [head][32 slots][head_dim] in one copy
     const flare_kv* kv_obj;           // the cache itself (tensor maps, ring state)
-    const int* h_attend;              // host copy of attend_len (valid during the call), or null
+    const int* h_attend = nullptr;    // host copy of attend_len (valid during the call), or null
+    const int2* h_ring = nullptr;     // host copy of ring, likewise
+    const StepFusion* fuse = nullptr;
     // defer_merge (with want_partial): the launcher leaves the per-range records unmerged and reports where they
     // are — [row][n_split][head_dim + 2], maximum in log2 units — so that the caller's own kernel merges them
     // (the multi-GPU exchange does, together with the records of the other ranks)
@@ -161,6 +180,9 @@ struct DecodeArgs {
     int* n_split_out = nullptr;
 };
 int flare_launch_decode(flare_attn_ctx* ctx, const DecodeArgs& a);
+// The per-sequence (position, length) and attend lengths on the device: uploaded when a kernel reads them there (the
+// Q8_0 kernel gets those of up to 64 sequences as launch parameters and needs no upload).
+int flare_small_on_device(flare_attn_ctx* ctx, const DecodeArgs& a, const int** d_attend, const int2** d_ring);
 int flare_launch_decode_generic(flare_attn_ctx* ctx, const DecodeArgs& a);
 bool flare_decode_q8_supported(const DecodeArgs& a);
 int flare_launch_decode_q8(flare_attn_ctx* ctx, const DecodeArgs& a);
@@ -185,7 +207,8 @@ int flare_launch_merge_splits(flare_attn_ctx* ctx, const float* work, int n_spli
                               int want_partial);
 extern "C" int flare_decode_common(flare_attn_ctx* ctx, flare_kv* kv, int layer, int num_heads, const float* q, int n_q,
                         const int* attend_len, float softcap, int slot_begin, int slot_end, int want_partial,
-                        int causal_q, float* out, int on_device, const float* q_staged = nullptr, int multi = 0);
+                        int causal_q, float* out, int on_device, const float* q_staged = nullptr, int multi = 0,
+                        const StepFusion* fuse = nullptr, size_t q_seq_stride = 0);
 
 struct PrefillArgs {
     const void *q, *k, *v; void* out;   // device

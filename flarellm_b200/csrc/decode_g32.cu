@@ -558,7 +558,8 @@ bool flare_decode_g32_supported(const DecodeArgs& a, const flare_kv* kv) {
 int flare_launch_decode_g32(flare_attn_ctx* ctx, const DecodeArgs& a, const flare_kv* kv) {
     const int nkv = a.kv.num_kv_heads, rows = a.batch * a.num_heads;
     G32Params p;
-    p.q = a.q; p.attend_len = a.attend_len; p.ring = a.ring;
+    p.q = a.q;
+    FLARE_TRY(flare_small_on_device(ctx, a, &p.attend_len, &p.ring));
     p.k_meta = reinterpret_cast<const unsigned char*>(a.kv.plane[FLARE_PLANE_K_SCALE]);
     p.v_meta = reinterpret_cast<const unsigned char*>(a.kv.plane[FLARE_PLANE_V_SCALE]);
     p.k_meta_seq_stride = a.kv.stride[FLARE_PLANE_K_SCALE];

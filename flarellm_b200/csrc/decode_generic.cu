@@ -440,7 +440,7 @@ int flare_launch_decode_generic(flare_attn_ctx* ctx, const DecodeArgs& a) {
     if (rows == 0) return FLARE_OK;
     DecodeParams p;
     p.kv = a.kv; p.q = a.q; p.out = a.out; p.work = nullptr;
-    p.attend_len = a.attend_len; p.ring = a.ring;
+    FLARE_TRY(flare_small_on_device(ctx, a, &p.attend_len, &p.ring));
     p.n_q = a.n_q; p.num_heads = a.num_heads;
     p.slot_begin = a.slot_begin; p.slot_end = a.slot_end; p.want_partial = a.want_partial; p.causal_q = a.causal_q;
     p.window = a.window;

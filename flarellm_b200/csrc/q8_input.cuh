@@ -20,14 +20,19 @@ __device__ __forceinline__ float flare_block_sum(float s, float* s_red) {
     return t;
 }
 
-// one warp, one block of 32 values (lane = element): amax, scale = amax / 127, q = round(n * (127 / amax)) as i8
-__device__ __forceinline__ void flare_quantize_block_of_32(float n, int lane, int8_t* q_out, float* s_out) {
+// One warp, one block of 32 values (lane = element): amax, scale = amax / 127, code = round(n * (127 / amax)) as i8.
+// Returns this lane's code; every lane gets the scale.
+__device__ __forceinline__ int flare_q8_code(float n, float& scale) {
     float amax = fabsf(n);
 #pragma unroll
     for (int off = 16; off; off >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, off));
-    const float scale = __fdiv_rn(amax, 127.0f);
+    scale = __fdiv_rn(amax, 127.0f);
     const float inv_scale = scale != 0.0f ? __fdiv_rn(127.0f, amax) : 0.0f;
-    q_out[lane] = flare_to_i8_saturating(roundf(__fmul_rn(n, inv_scale)));
+    return flare_to_i8_saturating(roundf(__fmul_rn(n, inv_scale)));
+}
+__device__ __forceinline__ void flare_quantize_block_of_32(float n, int lane, int8_t* q_out, float* s_out) {
+    float scale;
+    q_out[lane] = (int8_t)flare_q8_code(n, scale);
     if (lane == 0) *s_out = scale;
 }
 
