@@ -251,8 +251,29 @@ inline cudaError_t flare_launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 bl
 // matvec.cu: the two halves of flare_matvec_q8_0 on device buffers
 struct flare_weight;
 int flare_launch_quantize_input(flare_attn_ctx* ctx, const float* d_x, size_t n_blocks, int8_t* d_xq, float* d_xs);
-int flare_launch_matvec_q8_0_preq(flare_attn_ctx* ctx, const flare_weight* w, const int8_t* d_xq, const float* d_xs, int batch,
-                                  float* d_out, int accumulate);
+int flare_weight_upload(flare_attn_ctx* ctx, const void* blocks, int rows, int cols, int paired, flare_weight** out_w);
+// What a Q8_0 product reads: codes and scales, or f32 vectors that it quantises itself - as they are, after
+// rmsnorm_quantize_q8_0 ((x * norm) * inv_rms) or after rmsnorm_into ((x * inv_rms) * norm).
+enum { IN_CODES = 0, IN_F32 = 1, IN_NORM_Q8 = 2, IN_NORM_F32 = 3 };
+struct Q8Input {
+    int kind = IN_CODES;
+    const int8_t* xq = nullptr;      // [batch][cols]
+    const float* xs = nullptr;       // [batch][cols / 32]
+    const float* x = nullptr;        // [batch][cols], 16-byte aligned
+    const float* norm = nullptr;
+    float eps = 0.0f;
+};
+// What it writes: out = product, out += product (the residual connection), or - of a paired [gate | up] matrix -
+// silu(gate) * up as Q8_0 blocks.
+enum { OUT_F32 = 0, OUT_SILU_Q8 = 1 };
+struct Q8Output {
+    float* out = nullptr;            // [batch][rows]
+    int accumulate = 0;
+    int8_t* oq = nullptr;            // [batch][rows / 2]
+    float* os = nullptr;
+};
+bool flare_product_quantises(const flare_weight* w, int batch);       // the f32 input forms are there for this call
+int flare_launch_product_q8_0(flare_attn_ctx* ctx, const flare_weight* w, const Q8Input& in, int batch, const Q8Output& out);
 void flare_weight_dims(const flare_weight* w, int* rows, int* cols);
 int flare_launch_kv_export_dequant(flare_kv* kv, int layer, int seq, float* d_k, float* d_v);
 int flare_launch_q8_blocks(flare_kv* kv, int layer, int seq, int first_slot, int n_slots, void* d_kb, void* d_vb,

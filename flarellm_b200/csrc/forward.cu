@@ -22,6 +22,7 @@
 #include "common.cuh"
 #include "q8_input.cuh"
 
+#include <algorithm>
 #include <vector>
 
 struct flare_model {
@@ -38,9 +39,9 @@ struct flare_model {
     float* output_f32 = nullptr;
     // activations for `buf_batch` sequences
     int buf_batch = 0;
-    float *x = nullptr, *qkv = nullptr, *q = nullptr, *k = nullptr, *v = nullptr, *attn = nullptr, *proj = nullptr,
-          *gate_up = nullptr, *normed = nullptr, *logits = nullptr, *xs = nullptr;
-    int8_t* xq = nullptr;
+    float *x = nullptr, *qkv = nullptr, *q = nullptr, *k = nullptr, *v = nullptr, *attn = nullptr, *normed = nullptr,
+          *logits = nullptr, *xs = nullptr, *hs = nullptr;
+    int8_t *xq = nullptr, *hq = nullptr;             // quantised hidden-state inputs and feed-forward activations
     long long* pos = nullptr;        // the token's absolute positions, uploaded once per call
 };
 
@@ -50,8 +51,8 @@ namespace {
 __global__ void __launch_bounds__(256) rmsnorm_quantize_kernel(const float* __restrict__ x, const float* __restrict__ weight,
                                                                 float eps, int dim, int8_t* __restrict__ xq,
                                                                 float* __restrict__ xs) {
+    flare_pdl_trigger();      // a product, which requests weights before its own wait
     flare_pdl_wait();
-    flare_pdl_trigger();
     __shared__ float s_red[32];
     flare_quantize_vector(x + (size_t)blockIdx.x * dim, weight, eps, dim, xq + (size_t)blockIdx.x * dim,
                           xs + (size_t)blockIdx.x * (dim / 32), s_red);
@@ -91,27 +92,6 @@ __global__ void split_qkv_kernel(const float* __restrict__ qkv, int q_dim, int k
     }
 }
 
-// hidden = silu(gate) * up out of rows of [gate | up], quantised per 32 as quantize_input_q8_0 does: a warp per block
-__global__ void silu_mul_quantize_kernel(const float* __restrict__ gate_up, int inter, size_t n_blocks,
-                                         int8_t* __restrict__ xq, float* __restrict__ xs) {
-    flare_pdl_wait();
-    flare_pdl_trigger();
-    const int lane = threadIdx.x & 31, nb = inter / 32;
-    for (size_t w = (blockIdx.x * (size_t)blockDim.x + threadIdx.x) >> 5; w < n_blocks; w += ((size_t)gridDim.x * blockDim.x) >> 5) {
-        const size_t b = w / nb, blk = w % nb;
-        const float g = gate_up[b * 2 * inter + blk * 32 + lane];
-        const float u = gate_up[b * 2 * inter + inter + blk * 32 + lane];
-        const float h = __fmul_rn(__fdiv_rn(g, __fadd_rn(1.0f, expf(-g))), u);
-        float amax = fabsf(h);
-#pragma unroll
-        for (int off = 16; off; off >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, off));
-        const float d = __fdiv_rn(amax, 127.0f);
-        const float id = d != 0.0f ? __fdiv_rn(127.0f, amax) : 0.0f;
-        xq[w * 32 + lane] = flare_to_i8_saturating(roundf(__fmul_rn(h, id)));
-        if (lane == 0) xs[w] = d;
-    }
-}
-
 // f32 output matrix: a warp per row, the input vectors of the batch one after the other
 __global__ void __launch_bounds__(256) matvec_f32_kernel(const float* __restrict__ w, const float* __restrict__ x, int rows,
                                                          int cols, int batch, float* __restrict__ out) {
@@ -142,15 +122,16 @@ int upload_f32(flare_attn_ctx* ctx, const float* host, size_t n, float** dev) {
     return FLARE_OK;
 }
 
-int replace_weight(flare_attn_ctx* ctx, const void* blocks, int rows, int cols, flare_weight** slot) {
+int replace_weight(flare_attn_ctx* ctx, const void* blocks, int rows, int cols, flare_weight** slot, int paired = 0) {
     if (*slot) { flare_weight_free(*slot); *slot = nullptr; }
-    return flare_weight_upload_q8_0(ctx, blocks, rows, cols, slot);
+    return flare_weight_upload(ctx, blocks, rows, cols, paired, slot);
 }
 
 void free_buffers(flare_model* m) {
-    float** bufs[] = {&m->x, &m->qkv, &m->q, &m->k, &m->v, &m->attn, &m->proj, &m->gate_up, &m->normed, &m->logits, &m->xs};
+    float** bufs[] = {&m->x, &m->qkv, &m->q, &m->k, &m->v, &m->attn, &m->normed, &m->logits, &m->xs, &m->hs};
     for (float** b : bufs) { cudaFree(*b); *b = nullptr; }
     cudaFree(m->xq); m->xq = nullptr;
+    cudaFree(m->hq); m->hq = nullptr;
     cudaFree(m->pos); m->pos = nullptr;
     m->buf_batch = 0;
 }
@@ -162,15 +143,15 @@ int ensure_buffers(flare_model* m, int batch) {
     free_buffers(m);
     const flare_model_config& c = m->cfg;
     const size_t B = (size_t)batch, q_dim = (size_t)c.num_heads * c.head_dim, kv_dim = (size_t)c.num_kv_heads * c.head_dim;
-    const size_t widest = (size_t)(c.intermediate_dim > c.hidden_dim ? c.intermediate_dim : c.hidden_dim) > q_dim
-                              ? (size_t)(c.intermediate_dim > c.hidden_dim ? c.intermediate_dim : c.hidden_dim) : q_dim;
+    const size_t widest = std::max((size_t)c.hidden_dim, q_dim);
     struct { float** p; size_t n; } want[] = {
         {&m->x, B * c.hidden_dim}, {&m->qkv, B * (q_dim + 2 * kv_dim)}, {&m->q, B * q_dim}, {&m->k, B * kv_dim},
-        {&m->v, B * kv_dim}, {&m->attn, B * q_dim}, {&m->proj, B * c.hidden_dim}, {&m->gate_up, B * 2 * c.intermediate_dim},
-        {&m->normed, B * c.hidden_dim}, {&m->logits, B * c.vocab_size}, {&m->xs, B * widest / 32 + 8}};
+        {&m->v, B * kv_dim}, {&m->attn, B * q_dim}, {&m->normed, B * c.hidden_dim}, {&m->logits, B * c.vocab_size}, {&m->xs, B * widest / 32},
+        {&m->hs, B * c.intermediate_dim / 32}};
     for (auto& w : want)
         if (cudaMalloc((void**)w.p, w.n * sizeof(float)) != cudaSuccess) { cudaGetLastError(); free_buffers(m); return flare_set_error(ctx, FLARE_ERR_OOM, "forward buffers for %d sequences", batch); }
-    if (cudaMalloc((void**)&m->xq, B * widest) != cudaSuccess || cudaMalloc((void**)&m->pos, B * sizeof(long long)) != cudaSuccess) { cudaGetLastError(); free_buffers(m); return flare_set_error(ctx, FLARE_ERR_OOM, "forward buffers for %d sequences", batch); }
+    if (cudaMalloc((void**)&m->xq, B * widest) != cudaSuccess || cudaMalloc((void**)&m->hq, B * c.intermediate_dim) != cudaSuccess ||
+        cudaMalloc((void**)&m->pos, B * sizeof(long long)) != cudaSuccess) { cudaGetLastError(); free_buffers(m); return flare_set_error(ctx, FLARE_ERR_OOM, "forward buffers for %d sequences", batch); }
     m->buf_batch = batch;
     return FLARE_OK;
 }
@@ -218,7 +199,7 @@ int flare_model_set_layer(flare_model* m, int layer, const float* attn_norm, con
     FLARE_TRY(upload_f32(ctx, ffn_norm, c.hidden_dim, &L.ffn_norm));
     FLARE_TRY(replace_weight(ctx, qkv_q8_0, q_dim + 2 * kv_dim, c.hidden_dim, &L.qkv));
     FLARE_TRY(replace_weight(ctx, wo_q8_0, c.hidden_dim, q_dim, &L.wo));
-    FLARE_TRY(replace_weight(ctx, gate_up_q8_0, 2 * c.intermediate_dim, c.hidden_dim, &L.gate_up));
+    FLARE_TRY(replace_weight(ctx, gate_up_q8_0, 2 * c.intermediate_dim, c.hidden_dim, &L.gate_up, 1));
     FLARE_TRY(replace_weight(ctx, down_q8_0, c.hidden_dim, c.intermediate_dim, &L.down));
     return FLARE_OK;
 }
@@ -268,7 +249,7 @@ int flare_forward_token(flare_attn_ctx* ctx, flare_model* m, flare_kv* kv, const
     const int B = kv->batch;
     if (B > 256) return flare_set_error(ctx, FLARE_ERR_UNSUPPORTED, "flare_forward_token: %d sequences (at most 256)", B);
     FLARE_TRY(ensure_buffers(m, B));
-    const int dim = c.hidden_dim, inter = c.intermediate_dim, q_dim = c.num_heads * c.head_dim, kv_dim = c.num_kv_heads * c.head_dim;
+    const int dim = c.hidden_dim, q_dim = c.num_heads * c.head_dim, kv_dim = c.num_kv_heads * c.head_dim;
     cudaStream_t st = ctx->stream;
     // 256 threads, like a CTA of the matrix-vector kernel: the fused and the standalone norm add in the same order
     const int norm_threads = dim >= 256 ? 256 : 32 * (dim / 32);
@@ -280,38 +261,79 @@ int flare_forward_token(flare_attn_ctx* ctx, flare_model* m, flare_kv* kv, const
     FLARE_CUDA_OK(ctx, cudaMemcpyAsync(m->x, token_embed, (size_t)B * dim * sizeof(float), cudaMemcpyHostToDevice, st));
     FLARE_CUDA_OK(ctx, cudaMemcpyAsync(m->pos, positions, (size_t)B * sizeof(long long), cudaMemcpyHostToDevice, st));
     ctx->last_launch_overlappable = false;
-    // a single sequence needs no copy to take [q | k | v] apart
-    float* q = B == 1 ? m->qkv : m->q;
-    float* k = B == 1 ? m->qkv + q_dim : m->k;
-    float* v = B == 1 ? m->qkv + q_dim + kv_dim : m->v;
+    // Five launches a layer where the attention kernel takes [q | k | v] rows as they are (rotation, cache row, output as
+    // input blocks of the next product) and the products normalise the hidden state themselves (one sequence); what does
+    // not fit is a kernel of its own.
+    const int qkv_dim = q_dim + 2 * kv_dim;
+    DecodeArgs probe = {};
+    probe.kv = flare_layer_view(kv, 0);
+    probe.kmap = kv->has_maps ? &kv->kq_map : nullptr;
+    probe.n_q = 1; probe.num_heads = c.num_heads;
+    const bool fused_step = flare_decode_q8_supported(probe);
+    auto normed = [&](const flare_weight* w, const float* norm, Q8Input* in) -> int {
+        if (flare_product_quantises(w, B)) { in->kind = IN_NORM_Q8; in->x = m->x; in->norm = norm; in->eps = c.rms_norm_eps; return FLARE_OK; }
+        FLARE_CUDA_OK(ctx, flare_launch_pdl(rmsnorm_quantize_kernel, dim3(B), dim3(norm_threads), 0, st, m->x, norm, c.rms_norm_eps, dim, m->xq, m->xs));
+        FLARE_LAUNCH_CHECK(ctx);
+        in->xq = m->xq; in->xs = m->xs;
+        return FLARE_OK;
+    };
     for (int layer = 0; layer < c.num_layers; layer++) {
         const flare_model::Layer& L = m->layers[layer];
+        Q8Input in, attn_in, ffn_in, hidden;
+        Q8Output to_qkv, to_x, to_hidden;
+        to_qkv.out = m->qkv;
+        to_x.out = m->x; to_x.accumulate = 1;
+        to_hidden.oq = m->hq; to_hidden.os = m->hs;
+        hidden.xq = m->hq; hidden.xs = m->hs;
         // attention block
-        FLARE_CUDA_OK(ctx, flare_launch_pdl(rmsnorm_quantize_kernel, dim3(B), dim3(norm_threads), 0, st, m->x, L.attn_norm, c.rms_norm_eps, dim, m->xq, m->xs));
-        FLARE_LAUNCH_CHECK(ctx);
-        FLARE_TRY(flare_launch_matvec_q8_0_preq(ctx, L.qkv, m->xq, m->xs, B, m->qkv, 0));
-        if (B > 1) {
-            FLARE_CUDA_OK(ctx, flare_launch_pdl(split_qkv_kernel, dim3(grid_for((size_t)q_dim + 2 * kv_dim), B), dim3(256), 0, st, m->qkv, q_dim, kv_dim, m->q, m->k, m->v));
-            FLARE_LAUNCH_CHECK(ctx);
+        FLARE_TRY(normed(L.qkv, L.attn_norm, &in));
+        FLARE_TRY(flare_launch_product_q8_0(ctx, L.qkv, in, B, to_qkv));
+        bool quantised = false;
+        if (fused_step) {
+            StepFusion f;
+            f.k = m->qkv + q_dim; f.v = m->qkv + q_dim + kv_dim; f.row_stride = qkv_dim;
+            f.cos = kv->rope_cos; f.sin = kv->rope_sin; f.positions = m->pos;
+            f.oq = m->xq; f.os = m->xs; f.quantised = &quantised;
+            // no kernel since the upload above has stored rows of this layer: its tiles may be requested at once
+            ctx->last_launch_overlappable = true;
+            FLARE_TRY(flare_decode_common(ctx, kv, layer, c.num_heads, m->qkv, 1, nullptr, 0.0f, 0, -1, 0, 1, m->attn, 1, nullptr, 0, &f, qkv_dim));
+        } else {
+            float *q = m->qkv, *k = m->qkv + q_dim, *v = k + kv_dim;     // a single sequence needs no copy to take them apart
+            if (B > 1) {
+                q = m->q; k = m->k; v = m->v;
+                FLARE_CUDA_OK(ctx, flare_launch_pdl(split_qkv_kernel, dim3(grid_for((size_t)qkv_dim), B), dim3(256), 0, st, m->qkv, q_dim, kv_dim, q, k, v));
+                FLARE_LAUNCH_CHECK(ctx);
+            }
+            FLARE_TRY(flare_kv_write_step_rope_device(kv, layer, k, v, m->pos, q, c.num_heads));     // rotates q as well
+            FLARE_TRY(flare_decode_attn(ctx, kv, layer, c.num_heads, q, 1, nullptr, 0.0f, m->attn, 1));
         }
-        FLARE_TRY(flare_kv_write_step_rope_device(kv, layer, k, v, m->pos, q, c.num_heads));     // rotates q as well
-        FLARE_TRY(flare_decode_attn(ctx, kv, layer, c.num_heads, q, 1, nullptr, 0.0f, m->attn, 1));
-        FLARE_TRY(flare_launch_quantize_input(ctx, m->attn, (size_t)B * q_dim / 32, m->xq, m->xs));
-        FLARE_TRY(flare_launch_matvec_q8_0_preq(ctx, L.wo, m->xq, m->xs, B, m->x, 1));
+        if (quantised) { attn_in.xq = m->xq; attn_in.xs = m->xs; }
+        else if (flare_product_quantises(L.wo, B)) { attn_in.kind = IN_F32; attn_in.x = m->attn; }
+        else {
+            FLARE_TRY(flare_launch_quantize_input(ctx, m->attn, (size_t)B * q_dim / 32, m->xq, m->xs));
+            attn_in.xq = m->xq; attn_in.xs = m->xs;
+        }
+        FLARE_TRY(flare_launch_product_q8_0(ctx, L.wo, attn_in, B, to_x));
         // feed-forward block
-        FLARE_CUDA_OK(ctx, flare_launch_pdl(rmsnorm_quantize_kernel, dim3(B), dim3(norm_threads), 0, st, m->x, L.ffn_norm, c.rms_norm_eps, dim, m->xq, m->xs));
-        FLARE_LAUNCH_CHECK(ctx);
-        FLARE_TRY(flare_launch_matvec_q8_0_preq(ctx, L.gate_up, m->xq, m->xs, B, m->gate_up, 0));
-        FLARE_CUDA_OK(ctx, flare_launch_pdl(silu_mul_quantize_kernel, dim3(grid_for((size_t)B * inter)), dim3(256), 0, st, m->gate_up, inter, (size_t)B * inter / 32, m->xq, m->xs));
-        FLARE_LAUNCH_CHECK(ctx);
-        FLARE_TRY(flare_launch_matvec_q8_0_preq(ctx, L.down, m->xq, m->xs, B, m->x, 1));
-        ctx->last_launch_overlappable = false;
+        FLARE_TRY(normed(L.gate_up, L.ffn_norm, &ffn_in));
+        FLARE_TRY(flare_launch_product_q8_0(ctx, L.gate_up, ffn_in, B, to_hidden));
+        FLARE_TRY(flare_launch_product_q8_0(ctx, L.down, hidden, B, to_x));
     }
-    FLARE_CUDA_OK(ctx, flare_launch_pdl(rmsnorm_kernel, dim3(B), dim3(norm_threads), 0, st, m->x, m->output_norm, c.rms_norm_eps, dim, m->normed));
-    FLARE_LAUNCH_CHECK(ctx);
+    const bool fused_output = m->output_q8 && flare_product_quantises(m->output_q8, B);
+    if (!fused_output) {
+        FLARE_CUDA_OK(ctx, flare_launch_pdl(rmsnorm_kernel, dim3(B), dim3(norm_threads), 0, st, m->x, m->output_norm, c.rms_norm_eps, dim, m->normed));
+        FLARE_LAUNCH_CHECK(ctx);
+    }
     if (m->output_q8) {
-        FLARE_TRY(flare_launch_quantize_input(ctx, m->normed, (size_t)B * dim / 32, m->xq, m->xs));
-        FLARE_TRY(flare_launch_matvec_q8_0_preq(ctx, m->output_q8, m->xq, m->xs, B, m->logits, 0));
+        Q8Input in;
+        Q8Output to;
+        to.out = m->logits;
+        if (fused_output) { in.kind = IN_NORM_F32; in.x = m->x; in.norm = m->output_norm; in.eps = c.rms_norm_eps; }
+        else {
+            FLARE_TRY(flare_launch_quantize_input(ctx, m->normed, (size_t)B * dim / 32, m->xq, m->xs));
+            in.xq = m->xq; in.xs = m->xs;
+        }
+        FLARE_TRY(flare_launch_product_q8_0(ctx, m->output_q8, in, B, to));
     } else {
         FLARE_CUDA_OK(ctx, flare_launch_pdl(matvec_f32_kernel, dim3((c.vocab_size + 7) / 8), dim3(256), 0, st, m->output_f32, m->normed, c.vocab_size, dim, B, m->logits));
         FLARE_LAUNCH_CHECK(ctx);

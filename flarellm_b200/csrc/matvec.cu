@@ -1,4 +1,4 @@
-// Q8_0-weight matrix-vector products next to attention: the QKV projections before it and the output projection
+// Q8_0-weight matrix products next to attention: the QKV projections before it and the output projection
 // after it (flare-core/src/model.rs:2016-2136, 2249-2291), for `batch` input vectors at once.
 //
 // The arithmetic is the reference's, operation for operation, so that the result is the CPU's bit for bit
@@ -8,38 +8,60 @@
 //   matvec_q8_0_preq_into (8066-8100)   per row, blocks in ascending order:
 //                                       sum += (w_scale * x_scale[block]) * (int32 dot of the 32 int8 pairs) as f32
 //                                       with w_scale the block's f16 scale widened exactly; separate multiplies and add
-// The integer dot is exact in any order (dp4a); the f32 sum over a row's blocks is the only order-sensitive part and
-// is kept sequential: the lanes of a warp each own one input vector of the batch for that sum, so 32 sums run side
-// by side.  A weight row is read from HBM once for the whole batch.
+// The integer dot is exact in any order (one int8 MMA per block of 32); the f32 sum over a row's blocks is the only
+// order-sensitive part and stays sequential.
 #include "common.cuh"
 #include "q8_input.cuh"
 #include "tma.cuh"
+#include <algorithm>
 #include <mutex>
 
+// The GGUF block stream (f16 scale + 32 x i8 per 34 bytes) taken apart at upload into the order the product reads:
+// tiles of 16 rows, per tile its blocks in ascending order, per block BLK bytes: the 16 x 32 codes as the int8 MMA's A
+// operand (16 bytes per lane), then the 16 scales as (row g, row g + 8) pairs.  A run of blocks of a tile is one
+// contiguous piece on a 16-byte boundary whatever the width, and the bytes are the stream's own 34 per 32 values.
 struct flare_weight {
     flare_attn_ctx* ctx = nullptr;
     int rows = 0, cols = 0;
-    // the GGUF block stream (f16 LE scale + 32 x i8 per 34 bytes) taken apart at upload, so that the 32 weights
-    // of a block start on a 32-byte boundary: same numbers, same bytes per block read
-    int8_t* qs = nullptr;        // [rows][cols]
-    __half* sc = nullptr;        // [rows][cols / 32]
+    int paired = 0;              // rows are [gate | up]: tiles go gate 0-15, gate 16-31, up 0-15, up 16-31 of each 32 channels
+    unsigned char* packed = nullptr;
 };
 
 namespace {
 
-constexpr int CHUNK = 64;            // blocks of a row handled per pass: two per lane
-constexpr int WARPS = 8;
-constexpr int TS = CHUNK + 1;        // floats per input vector in the product buffer (odd: no bank conflicts in the sums)
+constexpr int BLK = 16 * 34;         // bytes of one block column of a tile
+constexpr int WARPS = 8;             // multiplying warps of a CTA
+constexpr int CHUNK = 64;            // blocks of a tile handled per step, at most: eight per warp
+constexpr int PER_WARP = CHUNK / WARPS;
+constexpr int MAX_STAGES = 8;
+constexpr int ROW1 = CHUNK + 8;      // floats per row of the one-vector kernel's products (8 extra: rows on other banks)
 
-// one thread per block: 34 bytes -> scale plane + weight plane
-__global__ void repack_q8_0_kernel(const unsigned char* __restrict__ blocks, size_t n_blocks, int8_t* __restrict__ qs,
-                                   __half* __restrict__ sc) {
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n_blocks; i += (size_t)gridDim.x * blockDim.x) {
-        const uint16_t* b16 = reinterpret_cast<const uint16_t*>(blocks + i * 34);
-        sc[i] = __ushort_as_half(b16[0]);
-        uint16_t* d16 = reinterpret_cast<uint16_t*>(qs + i * 32);
+// a thread per 16 bytes of the packed form: lane (g, t) of a block holds rows g and g + 8, channels 4t.. and 16 + 4t..
+__global__ void repack_q8_0_kernel(const unsigned char* __restrict__ blocks, int rows, int nb, int paired, size_t n_items,
+                                   unsigned char* __restrict__ packed) {
+    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n_items; i += (size_t)gridDim.x * blockDim.x) {
+        const int lane = (int)(i & 31), g = lane >> 2, t = lane & 3;
+        const size_t tb = i >> 5;
+        const int blk = (int)(tb % nb);
+        const size_t tile = tb / nb;
+        const size_t row0 = paired ? (tile >> 2) * 32 + (tile & 1) * 16 + ((tile >> 1) & 1) * (size_t)(rows / 2) : tile * 16;
+        unsigned char* dst = packed + tb * BLK;
+        uint32_t v[4];
 #pragma unroll
-        for (int j = 0; j < 16; j++) d16[j] = b16[1 + j];
+        for (int r = 0; r < 4; r++) {                 // a0: row g, a1: row g + 8, a2 / a3: the same, upper 16 channels
+            const size_t row = row0 + g + 8 * (r & 1);
+            v[r] = 0;
+            if (row < (size_t)rows) {
+                const uint16_t* s = reinterpret_cast<const uint16_t*>(blocks + (row * nb + blk) * 34) + 1 + 8 * (r >> 1) + 2 * t;
+                v[r] = (uint32_t)s[0] | (uint32_t)s[1] << 16;
+            }
+        }
+        *reinterpret_cast<uint4*>(dst + lane * 16) = make_uint4(v[0], v[1], v[2], v[3]);
+        if (t < 2) {
+            const size_t row = row0 + g + 8 * t;
+            *reinterpret_cast<uint16_t*>(dst + 512 + g * 4 + t * 2) =
+                row < (size_t)rows ? *reinterpret_cast<const uint16_t*>(blocks + (row * nb + blk) * 34) : (uint16_t)0;
+        }
     }
 }
 
@@ -53,306 +75,368 @@ __global__ void quantize_input_kernel(const float* __restrict__ x, size_t n_bloc
         flare_quantize_block_of_32(x[w * 32 + lane], lane, xq + w * 32, xs + w);
 }
 
-struct MatvecParams {
-    const int8_t* wq;            // [rows][cols]
-    const __half* ws;            // [rows][cols / 32]
-    const int8_t* xq;            // [batch][cols]
-    const float* xs;             // [batch][cols / 32]
-    float* out;                  // [batch][rows]
-    int rows, cols, batch;
-    int bt;                      // input vectors per tile: min(batch, 32); sizes the product buffer
-    int accumulate;              // out += product (the residual connection) instead of out = product
-    int* err;                    // status word of the context (a bulk copy that never arrives)
+struct ProductParams {
+    const unsigned char* w;
+    Q8Input in;
+    Q8Output out;
+    int rows, nb, batch;
+    int n_units;                 // tiles, or groups of four tiles of a paired matrix
+    int chunks, cb;              // steps per tile and blocks per step (the last one may have fewer)
+    int n_stages, stage_bytes;
+    int col_groups;              // groups of eight input vectors; neighbouring CTAs take the groups of the same tiles
+    int* err;
 };
 
-// A warp owns one row at a time.  Per chunk of 64 blocks every lane holds two blocks of the row in registers
-// (two 16-byte loads each, the warp reads 2 KB contiguous), multiplies them with every input vector of the tile
-// and leaves the products in shared memory; then lane b adds the chunk's products of input vector b in block order.
-__global__ void __launch_bounds__(32 * WARPS) matvec_q8_0_kernel(MatvecParams p) {
-    extern __shared__ __align__(16) float terms_all[];
-    flare_pdl_wait();
+__device__ __forceinline__ void mma_s8(int (&d)[4], const uint4& a, uint32_t b0, uint32_t b1, const int (&c)[4]) {
+    asm("mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%10, %11, %12, %13};"
+        : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3])
+        : "r"(a.x), "r"(a.y), "r"(a.z), "r"(a.w), "r"(b0), "r"(b1), "r"(c[0]), "r"(c[1]), "r"(c[2]), "r"(c[3]));
+}
+__device__ __forceinline__ float silu_mul(float gate, float up) {
+    return __fmul_rn(__fdiv_rn(gate, __fadd_rn(1.0f, expf(-gate))), up);
+}
+
+// Both kernels below walk steps of (16 rows) x (up to 64 blocks) of packed weights, 35 KB each, that one thread keeps
+// requesting as bulk copies into a ring.  In a step every warp multiplies its (up to) eight blocks by int8 MMAs, whose K
+// is exactly a block, and leaves the scaled products in shared memory; other threads add them in block order.
+//
+// What bounds them is HBM, and at a model's sizes (4 to 35 MB a matrix) the time until the first bytes arrive.  The
+// weights belong to no kernel of the stream, so the ring is filled before the wait for the predecessor, and the successor
+// is let in at once: its ring fills while this kernel works (two CTAs fit on an SM).  It reads nothing else before its
+// own wait.
+struct Steps {
+    int cta, n_cta, steps_per_unit, n_steps;
+    __device__ Steps(const ProductParams& p, int tiles) {
+        cta = blockIdx.x / p.col_groups; n_cta = gridDim.x / p.col_groups;
+        steps_per_unit = tiles * p.chunks;
+        n_steps = (cta < p.n_units ? (p.n_units - cta + n_cta - 1) / n_cta : 0) * steps_per_unit;
+    }
+};
+__device__ __forceinline__ void issue_step(const ProductParams& p, const Steps& st, int tiles, unsigned char* ring, uint64_t* bars, int s) {
+    const int unit = st.cta + s / st.steps_per_unit * st.n_cta, r = s % st.steps_per_unit, c0 = r % p.chunks * p.cb;
+    const size_t tile = (size_t)unit * tiles + r / p.chunks;
+    const uint32_t bytes = (uint32_t)min(p.cb, p.nb - c0) * BLK;
+    uint64_t* bar = &bars[s % p.n_stages];
+    ptx::mbar_expect_tx(bar, bytes);
+    ptx::bulk_load(ring + (size_t)(s % p.n_stages) * p.stage_bytes, p.w + (tile * p.nb + c0) * BLK, bytes, bar);
+}
+__device__ __forceinline__ void start_ring(const ProductParams& p, const Steps& st, int tiles, unsigned char* ring, uint64_t* bars) {
+    for (int s = 0; s < p.n_stages; s++) ptx::mbar_init(&bars[s], 1);
+    ptx::fence_barrier_init();
+    ptx::fence_proxy_async();
+    for (int s = 0; s < p.n_stages && s < st.n_steps; s++) issue_step(p, st, tiles, ring, bars, s);
+}
+// A copy never arrived: those in flight land (or give up) before the shared memory goes, and the host is told.
+__device__ __noinline__ void give_up(const ProductParams& p, const Steps& st, uint64_t* bars, int s) {
+    if (threadIdx.x != 0) return;
+    for (int k = s; k < s + p.n_stages && k < st.n_steps; k++) ptx::mbar_wait(&bars[k % p.n_stages], (uint32_t)((k / p.n_stages) & 1));
+    flare_report(p.err, FLARE_ERR_TIMEOUT);
+}
+
+// Up to eight input vectors (as codes): they are the MMA's eight columns.  128 threads add, one per (row, vector).
+template <int OUT>
+__global__ void __launch_bounds__(32 * WARPS, 2) product_q8_0_kernel(const ProductParams p) {
+    extern __shared__ __align__(128) unsigned char ring[];
+    __shared__ uint64_t full_bar[MAX_STAGES];
+    __shared__ float s_hid[8][33];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+    constexpr int TILES = OUT == OUT_SILU_Q8 ? 4 : 1;
+    float* terms = reinterpret_cast<float*>(ring + (size_t)p.n_stages * p.stage_bytes);
+    const int col0 = 8 * (blockIdx.x % p.col_groups);
+    const Steps st(p, TILES);
+    if (threadIdx.x == 0) start_ring(p, st, TILES, ring, full_bar);
     flare_pdl_trigger();
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int nb = p.cols / 32;
-    float* terms = terms_all + (size_t)warp * p.bt * TS;
-    const int n_tiles = (p.batch + 31) / 32;
-    const int8_t* xq = p.xq;
-    const float* xs = p.xs;
-    for (int row = blockIdx.x * WARPS + warp; row < p.rows; row += gridDim.x * WARPS) {
-        const int8_t* wrow = p.wq + (size_t)row * p.cols;
-        const __half* srow = p.ws + (size_t)row * nb;
-        float sum[8];                                 // running sums of this lane's input vector in each batch tile (batch <= 256)
+    flare_pdl_wait();
+
+    // B operand and scales of this warp's blocks of the current chunk: vector g's codes, the scales of vectors 2t, 2t + 1
+    uint32_t b[PER_WARP][2];
+    float xs[PER_WARP][2];
+    const int col = col0 + g;
+    auto load_codes = [&](int c0) {
+        const int cn = min(p.cb, p.nb - c0), per = (cn + WARPS - 1) / WARPS;
 #pragma unroll
-        for (int t = 0; t < 8; t++) sum[t] = 0.0f;
-        for (int c0 = 0; c0 < nb; c0 += CHUNK) {
-            const int cn = min(CHUNK, nb - c0);
-            // this lane's (up to) two blocks of the chunk
-            float wsc[2];
-            int4 w0[2], w1[2];
+        for (int j = 0; j < PER_WARP; j++) {
+            const int i = warp * per + j;
+            b[j][0] = b[j][1] = 0; xs[j][0] = xs[j][1] = 0.0f;
+            if (j < per && i < cn) {
+                if (col < p.batch) {
+                    const int8_t* src = p.in.xq + ((size_t)col * p.nb + c0 + i) * 32 + 4 * t;
+                    b[j][0] = *reinterpret_cast<const uint32_t*>(src);
+                    b[j][1] = *reinterpret_cast<const uint32_t*>(src + 16);
+                }
 #pragma unroll
-            for (int k = 0; k < 2; k++) {
-                const int blk = lane + 32 * k;
-                if (blk < cn) {
-                    const int4* wp = reinterpret_cast<const int4*>(wrow + (size_t)(c0 + blk) * 32);
-                    asm volatile("ld.global.nc.L1::no_allocate.v4.s32 {%0, %1, %2, %3}, [%4];"
-                                 : "=r"(w0[k].x), "=r"(w0[k].y), "=r"(w0[k].z), "=r"(w0[k].w) : "l"(wp));
-                    asm volatile("ld.global.nc.L1::no_allocate.v4.s32 {%0, %1, %2, %3}, [%4];"
-                                 : "=r"(w1[k].x), "=r"(w1[k].y), "=r"(w1[k].z), "=r"(w1[k].w) : "l"(wp + 1));
-                    wsc[k] = __half2float(srow[c0 + blk]);
-                } else {
-                    wsc[k] = 0.0f;
-                    w0[k] = make_int4(0, 0, 0, 0); w1[k] = make_int4(0, 0, 0, 0);
+                for (int k = 0; k < 2; k++)
+                    if (col0 + 2 * t + k < p.batch) xs[j][k] = p.in.xs[(size_t)(col0 + 2 * t + k) * p.nb + c0 + i];
+            }
+        }
+    };
+    load_codes(0);
+    __syncthreads();                                   // the barriers are initialised
+
+    // the (row, vector) whose sum this thread keeps (threads 0 .. 127): an accumulator register of lane tid / 4
+    const int srow = (threadIdx.x >> 4) + 8 * ((threadIdx.x >> 1) & 1), svec = 2 * ((threadIdx.x >> 2) & 3) + (threadIdx.x & 1);
+    const bool summing = threadIdx.x < 128 && col0 + svec < p.batch;
+    float sum = 0.0f, kept[TILES] = {};
+    const int none[4] = {0, 0, 0, 0};
+    for (int s = 0; s < st.n_steps; s++) {
+        const int stage = s % p.n_stages, r = s % st.steps_per_unit, chunk = r % p.chunks, c0 = chunk * p.cb;
+        const int unit = st.cta + s / st.steps_per_unit * st.n_cta, cn = min(p.cb, p.nb - c0), per = (cn + WARPS - 1) / WARPS;
+        const bool failed = !ptx::mbar_wait(&full_bar[stage], (uint32_t)((s / p.n_stages) & 1));
+        const unsigned char* buf = ring + (size_t)stage * p.stage_bytes;
+        auto scaled = [&](int i, const uint4& a, __half2 wsh, uint32_t b0, uint32_t b1, float xs0, float xs1) {
+            const float2 ws = __half22float2(wsh);
+            int d[4];
+            mma_s8(d, a, b0, b1, none);
+            float4 v;
+            v.x = __fmul_rn(__fmul_rn(ws.x, xs0), (float)d[0]);
+            v.y = __fmul_rn(__fmul_rn(ws.x, xs1), (float)d[1]);
+            v.z = __fmul_rn(__fmul_rn(ws.y, xs0), (float)d[2]);
+            v.w = __fmul_rn(__fmul_rn(ws.y, xs1), (float)d[3]);
+            *reinterpret_cast<float4*>(terms + FLARE_CK(i * 128 + lane * 4, 4, p.cb * 128, p.err)) = v;
+        };
+        if (cn == CHUNK) {                             // no bounds inside: the blocks' loads and MMAs run side by side
+            const unsigned char* mine = buf + warp * PER_WARP * BLK;
+            uint4 a[PER_WARP];
+            __half2 ws[PER_WARP];
+#pragma unroll
+            for (int j = 0; j < PER_WARP; j++) {
+                a[j] = *reinterpret_cast<const uint4*>(mine + j * BLK + lane * 16);
+                ws[j] = *reinterpret_cast<const __half2*>(mine + j * BLK + 512 + g * 4);
+            }
+#pragma unroll
+            for (int j = 0; j < PER_WARP; j++) scaled(warp * PER_WARP + j, a[j], ws[j], b[j][0], b[j][1], xs[j][0], xs[j][1]);
+        } else {
+#pragma unroll
+            for (int j = 0; j < PER_WARP; j++) {
+                const int i = warp * per + j;
+                if (j < per && i < cn) {
+                    const unsigned char* at = buf + FLARE_CK(i * BLK, BLK, p.stage_bytes, p.err);
+                    scaled(i, *reinterpret_cast<const uint4*>(at + lane * 16), *reinterpret_cast<const __half2*>(at + 512 + g * 4),
+                           b[j][0], b[j][1], xs[j][0], xs[j][1]);
                 }
             }
-#pragma unroll 1
-            for (int t = 0; t < n_tiles; t++) {
-                const int bn = min(32, p.batch - 32 * t);
-                __syncwarp();                         // the sums of the previous pass have read the buffer
-                for (int b = 0; b < bn; b++) {
-                    const size_t vec = (size_t)(32 * t + b);
+        }
+        if (p.chunks > 1 && s + 1 < st.n_steps) load_codes((s + 1) % p.chunks * p.cb);     // on their way during the sums
+        if (__syncthreads_or(failed)) { give_up(p, st, full_bar, s); return; }
+        // the products are there and the stage has been read
+        if (threadIdx.x == 0 && s + p.n_stages < st.n_steps) { ptx::fence_proxy_async(); issue_step(p, st, TILES, ring, full_bar, s + p.n_stages); }
+        if (threadIdx.x < 128) {
+            if (chunk == 0) sum = 0.0f;
+            if (summing) {
+                const float* tp = terms + threadIdx.x;
+                int i = 0;
+                for (; i + 16 <= cn; i += 16) {
+                    float v[16];
 #pragma unroll
-                    for (int k = 0; k < 2; k++) {
-                        const int blk = lane + 32 * k;
-                        if (blk < cn) {
-                            const int4* xp = reinterpret_cast<const int4*>(xq + vec * p.cols + (size_t)(c0 + blk) * 32);
-                            const int4 x0 = __ldg(xp), x1 = __ldg(xp + 1);
-                            int acc = 0;
-                            acc = __dp4a(w0[k].x, x0.x, acc); acc = __dp4a(w0[k].y, x0.y, acc);
-                            acc = __dp4a(w0[k].z, x0.z, acc); acc = __dp4a(w0[k].w, x0.w, acc);
-                            acc = __dp4a(w1[k].x, x1.x, acc); acc = __dp4a(w1[k].y, x1.y, acc);
-                            acc = __dp4a(w1[k].z, x1.z, acc); acc = __dp4a(w1[k].w, x1.w, acc);
-                            const float cs = __fmul_rn(wsc[k], __ldg(xs + vec * nb + c0 + blk));
-                            terms[b * TS + blk] = __fmul_rn(cs, (float)acc);
+                    for (int k = 0; k < 16; k++) v[k] = tp[(i + k) * 128];
+#pragma unroll
+                    for (int k = 0; k < 16; k++) sum = __fadd_rn(sum, v[k]);
+                }
+                for (; i < cn; i++) sum = __fadd_rn(sum, tp[i * 128]);
+            }
+            if (chunk == p.chunks - 1) {
+                if constexpr (OUT == OUT_SILU_Q8) {
+                    const int tile = r / p.chunks;
+#pragma unroll
+                    for (int k = 0; k < TILES; k++) if (k == tile) kept[k] = sum;
+                    if (tile == TILES - 1) {           // uniform over the CTA
+                        s_hid[svec][srow] = silu_mul(kept[0], kept[2]);
+                        s_hid[svec][16 + srow] = silu_mul(kept[1], kept[3]);
+                        asm volatile("bar.sync 1, 128;" ::: "memory");
+                        const int n_blocks = p.rows / 64;              // blocks of a hidden vector
+#pragma unroll
+                        for (int k = 0; k < 2; k++) {
+                            const int c = 2 * warp + k;
+                            if (col0 + c < p.batch) {
+                                const size_t at = (size_t)(col0 + c) * n_blocks + unit;
+                                flare_quantize_block_of_32(s_hid[c][lane], lane, p.out.oq + at * 32, p.out.os + at);
+                            }
                         }
                     }
-                }
-                __syncwarp();
-                // lane b adds the chunk's products of input vector b in block order
-                if (lane < bn) {
-                    float s = sum[t];
-                    const float* tp = terms + lane * TS;
-#pragma unroll 8
-                    for (int blk = 0; blk < cn; blk++) s = __fadd_rn(s, tp[blk]);
-                    sum[t] = s;
+                } else {
+                    const size_t out_row = (size_t)unit * 16 + srow;
+                    if (summing && out_row < (size_t)p.rows) {
+                        float* o = p.out.out + (size_t)(col0 + svec) * p.rows + out_row;
+                        *o = p.out.accumulate ? __fadd_rn(*o, sum) : sum;
+                    }
                 }
             }
         }
-#pragma unroll
-        for (int t = 0; t < 8; t++)
-            if (t < n_tiles && 32 * t + lane < p.batch) {
-                float* o = p.out + (size_t)(32 * t + lane) * p.rows + row;
-                *o = p.accumulate ? __fadd_rn(*o, sum[t]) : sum[t];
-            }
+        __syncthreads();                               // the sums have read the products
     }
 }
 
-// The same product with the weights staged through shared memory by bulk copies: every warp keeps a ring of
-// RING chunk buffers (64 blocks: 2 KB of weights + 128 B of scales) that lane 0 refills with cp.async.bulk as soon as
-// the warp has taken a chunk into registers, so several chunks per warp are on their way from HBM at any time without
-// costing registers.  Needs rows and chunks on 16-byte boundaries (cols % 256 == 0); used for one or two input vectors.
-constexpr int RING = 4;
-constexpr int RING_CHUNK_BYTES = CHUNK * 32 + CHUNK * 2;        // 2176
-
-__global__ void __launch_bounds__(32 * WARPS) matvec_q8_0_ring_kernel(MatvecParams p) {
-    extern __shared__ __align__(128) unsigned char ring_smem[];
-    __shared__ uint64_t full_bar[WARPS][RING];
-    flare_pdl_wait();
+// One input vector: the MMA's columns are eight consecutive blocks instead.  MMA j of a warp multiplies block j by its
+// input codes in column j and zeros elsewhere and adds to the same accumulators, so that eight MMAs leave 16 rows x 8
+// block dots, all of them wanted, for one round of scaling: a seventh of the instructions per step of a body like the
+// kernel's above with one column in use (which took 76 us for 128256 x 2048, issue bound; this one 45.7 = 6.1 TB/s).  A ninth warp adds, a lane per
+// row, while the others are at the next step.  The input's norm and quantisation run here while the first weights travel,
+// instead of in a kernel of their own.
+template <int IN, int OUT>
+__global__ void __launch_bounds__(32 * WARPS + 32, 2) product1_q8_0_kernel(const ProductParams p) {
+    extern __shared__ __align__(128) unsigned char ring[];
+    __shared__ uint64_t full_bar[MAX_STAGES];
+    __shared__ float s_sq[WARPS];
+    __shared__ uint32_t s_codes[IN == IN_CODES ? 1 : CHUNK * 8];
+    __shared__ float s_xs[IN == IN_CODES ? 1 : CHUNK];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+    constexpr int TILES = OUT == OUT_SILU_Q8 ? 4 : 1;
+    float* terms = reinterpret_cast<float*>(ring + (size_t)p.n_stages * p.stage_bytes);      // [2][16][ROW1]
+    const Steps st(p, TILES);
+    if (threadIdx.x == 0) start_ring(p, st, TILES, ring, full_bar);
     flare_pdl_trigger();
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int nb = p.cols / 32;
-    const int chunks_per_row = (nb + CHUNK - 1) / CHUNK;
-    unsigned char* my_ring = ring_smem + (size_t)warp * RING * RING_CHUNK_BYTES;
-    float* terms = reinterpret_cast<float*>(ring_smem + (size_t)WARPS * RING * RING_CHUNK_BYTES) + (size_t)warp * p.bt * TS;
-    uint64_t* bars = full_bar[warp];
-    // this warp's rows: first_row, first_row + row_step, ...; its units are (row, chunk) pairs in that order
-    const int first_row = blockIdx.x * WARPS + warp, row_step = gridDim.x * WARPS;
-    const int my_rows = first_row < p.rows ? (p.rows - first_row + row_step - 1) / row_step : 0;
-    const long long n_units = (long long)my_rows * chunks_per_row;
-    auto issue = [&](long long u) {                    // lane 0 only
-        const int s = (int)(u % RING);
-        const int row = first_row + (int)(u / chunks_per_row) * row_step, c0 = (int)(u % chunks_per_row) * CHUNK;
-        const int cn = min(CHUNK, nb - c0);
-        unsigned char* dst = my_ring + (size_t)s * RING_CHUNK_BYTES;
-        ptx::mbar_expect_tx(&bars[s], (uint32_t)cn * 34);
-        ptx::bulk_load(dst, p.wq + (size_t)row * p.cols + (size_t)c0 * 32, (uint32_t)cn * 32, &bars[s]);
-        ptx::bulk_load(dst + CHUNK * 32, p.ws + (size_t)row * nb + c0, (uint32_t)cn * 2, &bars[s]);
-    };
-    if (lane == 0) {
-        for (int s = 0; s < RING; s++) ptx::mbar_init(&bars[s], 1);
-        ptx::fence_barrier_init();
-        ptx::fence_proxy_async();
-        for (long long u = 0; u < RING && u < n_units; u++) issue(u);
-    }
-    __syncwarp();
-    float sum = 0.0f;                                  // lane b: running sum of input vector b for the current row
-    bool failed = false;
-    for (long long u = 0; u < n_units; u++) {
-        const int s = (int)(u % RING);
-        const int row = first_row + (int)(u / chunks_per_row) * row_step, chunk = (int)(u % chunks_per_row), c0 = chunk * CHUNK;
-        const int cn = min(CHUNK, nb - c0);
-        if (!ptx::mbar_wait(&bars[s], (uint32_t)((u / RING) & 1))) { failed = true; break; }
-        const unsigned char* buf = my_ring + (size_t)s * RING_CHUNK_BYTES;
-        float wsc[2];
-        int4 w0[2], w1[2];
+    flare_pdl_wait();
+
+    if constexpr (IN != IN_CODES) {                    // one chunk: p.nb <= CHUNK
+        float inv_rms = 1.0f;
+        if constexpr (IN != IN_F32) {                  // the sum of squares in the order of the norm kernels
+            if (warp < WARPS) {
+                float e[PER_WARP], sq = 0.0f;
 #pragma unroll
-        for (int k = 0; k < 2; k++) {
-            const int blk = lane + 32 * k;
-            if (blk < cn) {
-                const int4* wp = reinterpret_cast<const int4*>(buf + blk * 32);
-                w0[k] = wp[0]; w1[k] = wp[1];
-                wsc[k] = __half2float(*reinterpret_cast<const __half*>(buf + CHUNK * 32 + blk * 2));
-            } else {
-                wsc[k] = 0.0f; w0[k] = make_int4(0, 0, 0, 0); w1[k] = make_int4(0, 0, 0, 0);
+                for (int k = 0; k < PER_WARP; k++) e[k] = warp + WARPS * k < p.nb ? p.in.x[(warp + WARPS * k) * 32 + lane] : 0.0f;
+#pragma unroll
+                for (int k = 0; k < PER_WARP; k++) sq = fmaf(e[k], e[k], sq);
+#pragma unroll
+                for (int off = 16; off; off >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, off);
+                if (lane == 0) s_sq[warp] = sq;
             }
-        }
-        __syncwarp();                                  // every lane has its blocks: the buffer may be refilled
-        if (lane == 0 && u + RING < n_units) { ptx::fence_proxy_async(); issue(u + RING); }
-        for (int b = 0; b < p.batch; b++) {
+            __syncthreads();
+            float sum = 0.0f;
 #pragma unroll
-            for (int k = 0; k < 2; k++) {
-                const int blk = lane + 32 * k;
-                if (blk < cn) {
-                    const int4* xp = reinterpret_cast<const int4*>(p.xq + (size_t)b * p.cols + (size_t)(c0 + blk) * 32);
-                    const int4 x0 = __ldg(xp), x1 = __ldg(xp + 1);
-                    int acc = 0;
-                    acc = __dp4a(w0[k].x, x0.x, acc); acc = __dp4a(w0[k].y, x0.y, acc);
-                    acc = __dp4a(w0[k].z, x0.z, acc); acc = __dp4a(w0[k].w, x0.w, acc);
-                    acc = __dp4a(w1[k].x, x1.x, acc); acc = __dp4a(w1[k].y, x1.y, acc);
-                    acc = __dp4a(w1[k].z, x1.z, acc); acc = __dp4a(w1[k].w, x1.w, acc);
-                    const float cs = __fmul_rn(wsc[k], __ldg(p.xs + (size_t)b * nb + c0 + blk));
-                    terms[b * TS + blk] = __fmul_rn(cs, (float)acc);
+            for (int w = 0; w < WARPS; w++) sum += s_sq[w];
+            inv_rms = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(sum, (float)(p.nb * 32)), p.in.eps)));
+        }
+        // four values per lane, eight lanes per block
+        for (int u = threadIdx.x; u < (p.nb * 8 + 31) / 32 * 32; u += 32 * WARPS + 32) {
+            float n[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+            if (u < p.nb * 8) {
+                const float4 xv = *reinterpret_cast<const float4*>(p.in.x + 4 * u);
+                n[0] = xv.x; n[1] = xv.y; n[2] = xv.z; n[3] = xv.w;
+                if constexpr (IN != IN_F32) {          // the two norms of the CPU multiply in different order
+                    const float4 nv = __ldg(reinterpret_cast<const float4*>(p.in.norm + 4 * u));
+                    const float nw[4] = {nv.x, nv.y, nv.z, nv.w};
+#pragma unroll
+                    for (int i = 0; i < 4; i++)
+                        n[i] = IN == IN_NORM_Q8 ? __fmul_rn(__fmul_rn(n[i], nw[i]), inv_rms) : __fmul_rn(__fmul_rn(n[i], inv_rms), nw[i]);
                 }
             }
+            float amax = fmaxf(fmaxf(fabsf(n[0]), fabsf(n[1])), fmaxf(fabsf(n[2]), fabsf(n[3])));
+#pragma unroll
+            for (int off = 4; off; off >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, off));
+            const float d = __fdiv_rn(amax, 127.0f), id = d != 0.0f ? __fdiv_rn(127.0f, amax) : 0.0f;
+            uint32_t c = 0;
+#pragma unroll
+            for (int i = 0; i < 4; i++) c |= (uint32_t)(uint8_t)flare_to_i8_saturating(roundf(__fmul_rn(n[i], id))) << (8 * i);
+            if (u < p.nb * 8) {
+                s_codes[u] = c;
+                if ((u & 7) == 0) s_xs[u >> 3] = d;
+            }
         }
-        __syncwarp();
-        if (lane < p.batch) {
+    }
+    __syncthreads();                                   // the codes are there, the barriers initialised
+
+    if (warp == WARPS) {                               // the adding warp: lane = row
+        float sum = 0.0f, kept[TILES] = {};
+        for (int s = 0; s < st.n_steps; s++) {
+            const int r = s % st.steps_per_unit, chunk = r % p.chunks, cn = min(p.cb, p.nb - chunk * p.cb);
+            const int unit = st.cta + s / st.steps_per_unit * st.n_cta;
+            if (__syncthreads_or(0)) return;
+            const float* tp = terms + (s & 1) * 16 * ROW1 + (lane & 15) * ROW1;
             if (chunk == 0) sum = 0.0f;
-            const float* tp = terms + lane * TS;
-#pragma unroll 8
-            for (int blk = 0; blk < cn; blk++) sum = __fadd_rn(sum, tp[blk]);
-            if (chunk == chunks_per_row - 1) {
-                float* o = p.out + (size_t)lane * p.rows + row;
-                *o = p.accumulate ? __fadd_rn(*o, sum) : sum;
+            int i = 0;
+            for (; i + 16 <= cn; i += 16) {
+                float4 v[4];
+#pragma unroll
+                for (int k = 0; k < 4; k++) v[k] = *reinterpret_cast<const float4*>(tp + i + 4 * k);
+#pragma unroll
+                for (int k = 0; k < 4; k++) sum = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(sum, v[k].x), v[k].y), v[k].z), v[k].w);
+            }
+            for (; i < cn; i++) sum = __fadd_rn(sum, tp[i]);
+            if (chunk != p.chunks - 1) continue;
+            if constexpr (OUT == OUT_SILU_Q8) {
+                const int tile = r / p.chunks;
+#pragma unroll
+                for (int k = 0; k < TILES; k++) if (k == tile) kept[k] = sum;
+                if (tile == TILES - 1) {               // lanes 16 .. 31 hold the same sums as 0 .. 15
+                    const float h = lane < 16 ? silu_mul(kept[0], kept[2]) : silu_mul(kept[1], kept[3]);
+                    flare_quantize_block_of_32(h, lane, p.out.oq + (size_t)unit * 32, p.out.os + unit);
+                }
+            } else {
+                const size_t row = (size_t)unit * 16 + lane;
+                if (lane < 16 && row < (size_t)p.rows) p.out.out[row] = p.out.accumulate ? __fadd_rn(p.out.out[row], sum) : sum;
             }
         }
-        __syncwarp();                                  // the sums have read the products before the next chunk writes them
+        return;
     }
-    if (failed && lane == 0) flare_report(p.err, FLARE_ERR_TIMEOUT);
-}
 
-// One input vector, rows of at most 64 blocks (cols <= 2048: the projections that read the hidden state): the case a
-// single-token forward pass spends most of its bytes on.  Two things change against the kernel above.  The input's
-// blocks of a lane are the same for every row, so they stay in registers for the whole kernel; and the ordered sum of
-// a row, which one lane has to do alone, is done for GROUP rows at a time, a lane per row, so that its 64 dependent
-// adds cost 8 instruction slots per row instead of 128.
-constexpr int GROUP = 16;
-
-__global__ void __launch_bounds__(32 * WARPS) matvec_q8_0_ring1_kernel(MatvecParams p) {
-    extern __shared__ __align__(128) unsigned char ring_smem[];
-    __shared__ uint64_t full_bar[WARPS][RING];
-    flare_pdl_wait();
-    flare_pdl_trigger();
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int nb = p.cols / 32;                       // <= 64: one chunk per row
-    unsigned char* my_ring = ring_smem + (size_t)warp * RING * RING_CHUNK_BYTES;
-    float* terms = reinterpret_cast<float*>(ring_smem + (size_t)WARPS * RING * RING_CHUNK_BYTES) + (size_t)warp * GROUP * TS;
-    uint64_t* bars = full_bar[warp];
-    const int first_row = blockIdx.x * WARPS + warp, row_step = gridDim.x * WARPS;
-    const int my_rows = first_row < p.rows ? (p.rows - first_row + row_step - 1) / row_step : 0;
-    auto issue = [&](int k) {                          // lane 0 only: row number k of this warp -> stage k % RING
-        const int s = k % RING;
-        const int row = first_row + k * row_step;
-        unsigned char* dst = my_ring + (size_t)s * RING_CHUNK_BYTES;
-        ptx::mbar_expect_tx(&bars[s], (uint32_t)nb * 34);
-        ptx::bulk_load(dst, p.wq + (size_t)row * p.cols, (uint32_t)nb * 32, &bars[s]);
-        ptx::bulk_load(dst + CHUNK * 32, p.ws + (size_t)row * nb, (uint32_t)nb * 2, &bars[s]);
+    // lane (g, t): codes of block g of this warp's eight, scales of blocks 2t and 2t + 1
+    uint32_t b0, b1;
+    float xs0, xs1;
+    auto load_codes = [&](int c0) {
+        const int cn = min(p.cb, p.nb - c0), i = warp * 8;
+        b0 = b1 = 0; xs0 = xs1 = 0.0f;
+        const uint32_t* codes = IN == IN_CODES ? reinterpret_cast<const uint32_t*>(p.in.xq) : s_codes;
+        const float* scales = IN == IN_CODES ? p.in.xs : s_xs;
+        if (i + g < cn) { b0 = codes[(c0 + i + g) * 8 + t]; b1 = codes[(c0 + i + g) * 8 + 4 + t]; }
+        if (i + 2 * t < cn) xs0 = scales[c0 + i + 2 * t];
+        if (i + 2 * t + 1 < cn) xs1 = scales[c0 + i + 2 * t + 1];
     };
-    if (lane == 0) {
-        for (int s = 0; s < RING; s++) ptx::mbar_init(&bars[s], 1);
-        ptx::fence_barrier_init();
-        ptx::fence_proxy_async();
-        for (int k = 0; k < RING && k < my_rows; k++) issue(k);
-    }
-    // the input's blocks of this lane
-    int4 x0[2], x1[2];
-    float xsc[2];
+    load_codes(0);
+    for (int s = 0; s < st.n_steps; s++) {
+        const int stage = s % p.n_stages, chunk = s % p.chunks, cn = min(p.cb, p.nb - chunk * p.cb);
+        const bool failed = !ptx::mbar_wait(&full_bar[stage], (uint32_t)((s / p.n_stages) & 1));
+        const int n = min(8, cn - warp * 8);           // this warp's blocks (none or fewer: none)
+        if (n > 0) {
+            const unsigned char* mine = ring + FLARE_CK((uint32_t)stage * p.stage_bytes + warp * 8 * BLK, n * BLK, p.n_stages * p.stage_bytes, p.err);
+            int d[2][4] = {};                          // two chains
+            float2 w0 = make_float2(0.0f, 0.0f), w1 = w0;
+            if (n == 8) {
+                uint4 a[8];
 #pragma unroll
-    for (int k = 0; k < 2; k++) {
-        const int blk = lane + 32 * k;
-        if (blk < nb) {
-            const int4* xp = reinterpret_cast<const int4*>(p.xq + (size_t)blk * 32);
-            x0[k] = __ldg(xp); x1[k] = __ldg(xp + 1);
-            xsc[k] = __ldg(p.xs + blk);
-        } else {
-            x0[k] = make_int4(0, 0, 0, 0); x1[k] = make_int4(0, 0, 0, 0); xsc[k] = 0.0f;
-        }
-    }
-    __syncwarp();
-    bool failed = false;
-    for (int k = 0; k < my_rows; k++) {
-        const int s = k % RING, slot = k % GROUP;
-        if (!ptx::mbar_wait(&bars[s], (uint32_t)((k / RING) & 1))) { failed = true; break; }
-        const unsigned char* buf = my_ring + (size_t)s * RING_CHUNK_BYTES;
-        float t[2];
+                for (int j = 0; j < 8; j++) a[j] = *reinterpret_cast<const uint4*>(mine + j * BLK + lane * 16);
 #pragma unroll
-        for (int j = 0; j < 2; j++) {
-            const int blk = lane + 32 * j;
-            if (blk < nb) {
-                const int4* wp = reinterpret_cast<const int4*>(buf + blk * 32);
-                const int4 w0 = wp[0], w1 = wp[1];
-                const float wsc = __half2float(*reinterpret_cast<const __half*>(buf + CHUNK * 32 + blk * 2));
-                int acc = 0;
-                acc = __dp4a(w0.x, x0[j].x, acc); acc = __dp4a(w0.y, x0[j].y, acc);
-                acc = __dp4a(w0.z, x0[j].z, acc); acc = __dp4a(w0.w, x0[j].w, acc);
-                acc = __dp4a(w1.x, x1[j].x, acc); acc = __dp4a(w1.y, x1[j].y, acc);
-                acc = __dp4a(w1.z, x1[j].z, acc); acc = __dp4a(w1.w, x1[j].w, acc);
-                t[j] = __fmul_rn(__fmul_rn(wsc, xsc[j]), (float)acc);
-            } else t[j] = 0.0f;
-        }
-        __syncwarp();                                  // every lane has read its blocks: the buffer may be refilled
-        if (lane == 0 && k + RING < my_rows) { ptx::fence_proxy_async(); issue(k + RING); }
-        if (lane < nb) terms[slot * TS + lane] = t[0];
-        if (lane + 32 < nb) terms[slot * TS + lane + 32] = t[1];
-        if (slot == GROUP - 1 || k == my_rows - 1) {
-            __syncwarp();
-            if (lane <= slot) {                        // lane r: the r-th row of this group, blocks in ascending order
-                const float* tp = terms + lane * TS;
-                float sum = 0.0f;
-#pragma unroll 8
-                for (int blk = 0; blk < nb; blk++) sum = __fadd_rn(sum, tp[blk]);
-                float* o = p.out + (first_row + (k - slot + lane) * row_step);
-                *o = p.accumulate ? __fadd_rn(*o, sum) : sum;
+                for (int j = 0; j < 8; j++) mma_s8(d[j & 1], a[j], g == j ? b0 : 0u, g == j ? b1 : 0u, d[j & 1]);
+            } else {
+#pragma unroll
+                for (int j = 0; j < 7; j++)
+                    if (j < n) mma_s8(d[j & 1], *reinterpret_cast<const uint4*>(mine + j * BLK + lane * 16), g == j ? b0 : 0u, g == j ? b1 : 0u, d[j & 1]);
             }
-            __syncwarp();
+            if (2 * t < n) w0 = __half22float2(*reinterpret_cast<const __half2*>(mine + 2 * t * BLK + 512 + g * 4));
+            if (2 * t + 1 < n) w1 = __half22float2(*reinterpret_cast<const __half2*>(mine + (2 * t + 1) * BLK + 512 + g * 4));
+            float* row = terms + (s & 1) * 16 * ROW1 + g * ROW1 + warp * 8 + 2 * t;
+            *reinterpret_cast<float2*>(row) = make_float2(__fmul_rn(__fmul_rn(w0.x, xs0), (float)(d[0][0] + d[1][0])),
+                                                          __fmul_rn(__fmul_rn(w1.x, xs1), (float)(d[0][1] + d[1][1])));
+            *reinterpret_cast<float2*>(row + 8 * ROW1) = make_float2(__fmul_rn(__fmul_rn(w0.y, xs0), (float)(d[0][2] + d[1][2])),
+                                                                     __fmul_rn(__fmul_rn(w1.y, xs1), (float)(d[0][3] + d[1][3])));
         }
+        if (p.chunks > 1 && s + 1 < st.n_steps) load_codes((s + 1) % p.chunks * p.cb);
+        if (__syncthreads_or(failed)) { give_up(p, st, full_bar, s); return; }
+        if (threadIdx.x == 0 && s + p.n_stages < st.n_steps) { ptx::fence_proxy_async(); issue_step(p, st, TILES, ring, full_bar, s + p.n_stages); }
     }
-    if (failed && lane == 0) flare_report(p.err, FLARE_ERR_TIMEOUT);
 }
 
 }  // namespace
 
-extern "C" {
-
-int flare_weight_upload_q8_0(flare_attn_ctx* ctx, const void* blocks, int rows, int cols, flare_weight** out_w) {
+// paired: the rows are [gate | up] halves of a feed-forward matrix (rows a multiple of 64)
+int flare_weight_upload(flare_attn_ctx* ctx, const void* blocks, int rows, int cols, int paired, flare_weight** out_w) {
     if (!ctx) return FLARE_ERR_INVALID_ARG;
     if (!out_w) return flare_set_error(ctx, FLARE_ERR_INVALID_ARG, "out_w is null");
     *out_w = nullptr;
-    if (!blocks || rows < 1 || cols < 32 || cols % 32)
+    if (!blocks || rows < 1 || cols < 32 || cols % 32 || (paired && rows % 64))
         return flare_set_error(ctx, FLARE_ERR_INVALID_ARG, "flare_weight_upload_q8_0: %d x %d (cols must be a positive multiple of 32)", rows, cols);
     FLARE_CUDA_OK(ctx, cudaSetDevice(ctx->device));
     flare_weight* w = new (std::nothrow) flare_weight();
     if (!w) return FLARE_ERR_OOM;
-    w->ctx = ctx; w->rows = rows; w->cols = cols;
-    const size_t n_blocks = (size_t)rows * (cols / 32), bytes = n_blocks * 34;
+    w->ctx = ctx; w->rows = rows; w->cols = cols; w->paired = paired;
+    const int nb = cols / 32;
+    const size_t tile_blocks = (size_t)((rows + 15) / 16) * nb, bytes = (size_t)rows * nb * 34;
     unsigned char* raw = nullptr;
-    cudaError_t e = cudaMalloc(&raw, bytes + 64);
-    if (e == cudaSuccess) e = cudaMalloc(&w->qs, n_blocks * 32);
-    if (e == cudaSuccess) e = cudaMalloc(&w->sc, n_blocks * sizeof(__half));
+    cudaError_t e = cudaMalloc(&raw, bytes);
+    if (e == cudaSuccess) e = cudaMalloc(&w->packed, tile_blocks * BLK);
     if (e == cudaSuccess) e = cudaMemcpyAsync(raw, blocks, bytes, cudaMemcpyHostToDevice, ctx->stream);
     if (e == cudaSuccess) {
-        size_t g = (n_blocks + 255) / 256;
-        if (g > 148 * 32) g = 148 * 32;
-        repack_q8_0_kernel<<<(int)g, 256, 0, ctx->stream>>>(raw, n_blocks, w->qs, w->sc);
+        const size_t g = std::min<size_t>((tile_blocks * 32 + 255) / 256, 148 * 32);
+        repack_q8_0_kernel<<<(int)g, 256, 0, ctx->stream>>>(raw, rows, nb, paired, tile_blocks * 32, w->packed);
         e = cudaGetLastError();
     }
     if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
@@ -361,7 +445,7 @@ int flare_weight_upload_q8_0(flare_attn_ctx* ctx, const void* blocks, int rows, 
         const int code = e == cudaErrorMemoryAllocation ? FLARE_ERR_OOM : FLARE_ERR_CUDA;
         flare_set_error(ctx, code, "flare_weight_upload_q8_0: %zu bytes: %s", bytes, cudaGetErrorString(e));
         cudaGetLastError();
-        cudaFree(w->qs); cudaFree(w->sc);
+        cudaFree(w->packed);
         delete w;
         return code;
     }
@@ -369,11 +453,17 @@ int flare_weight_upload_q8_0(flare_attn_ctx* ctx, const void* blocks, int rows, 
     return FLARE_OK;
 }
 
+extern "C" {
+
+int flare_weight_upload_q8_0(flare_attn_ctx* ctx, const void* blocks, int rows, int cols, flare_weight** out_w) {
+    return flare_weight_upload(ctx, blocks, rows, cols, 0, out_w);
+}
+
 int flare_weight_free(flare_weight* w) {
     if (!w) return FLARE_OK;
     cudaSetDevice(w->ctx->device);
     cudaStreamSynchronize(w->ctx->stream);
-    cudaFree(w->qs); cudaFree(w->sc);
+    cudaFree(w->packed);
     delete w;
     return FLARE_OK;
 }
@@ -397,8 +487,15 @@ int flare_matvec_q8_0(flare_attn_ctx* ctx, const flare_weight* w, const float* x
         FLARE_CUDA_OK(ctx, cudaMemcpyAsync(d + x_off, x, xn * 4, cudaMemcpyHostToDevice, ctx->stream));
         dx = (const float*)(d + x_off); dout = (float*)(d + o_off);
     }
-    FLARE_TRY(flare_launch_quantize_input(ctx, dx, nblk, (int8_t*)(d + q_off), (float*)(d + s_off)));
-    FLARE_TRY(flare_launch_matvec_q8_0_preq(ctx, w, (const int8_t*)(d + q_off), (const float*)(d + s_off), batch, dout, 0));
+    Q8Input in;
+    Q8Output to;
+    to.out = dout;
+    if (flare_product_quantises(w, batch) && ((uintptr_t)dx & 15) == 0) { in.kind = IN_F32; in.x = dx; }
+    else {
+        FLARE_TRY(flare_launch_quantize_input(ctx, dx, nblk, (int8_t*)(d + q_off), (float*)(d + s_off)));
+        in.xq = (const int8_t*)(d + q_off); in.xs = (const float*)(d + s_off);
+    }
+    FLARE_TRY(flare_launch_product_q8_0(ctx, w, in, batch, to));
     if (!on_device) {
         FLARE_CUDA_OK(ctx, cudaMemcpyAsync(out, dout, on * 4, cudaMemcpyDeviceToHost, ctx->stream));
         FLARE_CUDA_OK(ctx, cudaStreamSynchronize(ctx->stream));
@@ -420,75 +517,53 @@ int flare_launch_quantize_input(flare_attn_ctx* ctx, const float* d_x, size_t n_
     return FLARE_OK;
 }
 
-// matvec_q8_0_preq_into for `batch` quantised input vectors, all on the device; accumulate: out += product (the
-// residual connection) instead of out = product.  (Letting every CTA quantise the f32 input for itself, to save the
-// quantiser's launch, was measured slower: 1.69 instead of 1.55 ms per token of the 1B-shaped forward pass.)
-int flare_launch_matvec_q8_0_preq(flare_attn_ctx* ctx, const flare_weight* w, const int8_t* d_xq, const float* d_xs, int batch,
-                                  float* d_out, int accumulate) {
-    MatvecParams p;
-    p.wq = w->qs; p.ws = w->sc; p.xq = d_xq; p.xs = d_xs; p.out = d_out;
-    p.rows = w->rows; p.cols = w->cols; p.batch = batch;
-    p.bt = batch < 32 ? batch : 32;
-    p.accumulate = accumulate;
-    const int smem = WARPS * p.bt * TS * (int)sizeof(float);
+// One vector of at most 64 blocks is quantised by the product itself.  (With eight vectors each CTA would spend 9 us on
+// what a kernel of its own does in 2.5, most of it hidden behind the first weights.)
+bool flare_product_quantises(const flare_weight* w, int batch) { return batch == 1 && w->cols <= CHUNK * 32; }
+
+using ProductKernel = void (*)(const ProductParams);
+static ProductKernel product_kernel(int in, int out, bool one) {
+    if (!one) return out == OUT_SILU_Q8 ? product_q8_0_kernel<OUT_SILU_Q8> : product_q8_0_kernel<OUT_F32>;
+    if (out == OUT_SILU_Q8) return in == IN_CODES ? product1_q8_0_kernel<IN_CODES, OUT_SILU_Q8> : product1_q8_0_kernel<IN_NORM_Q8, OUT_SILU_Q8>;
+    switch (in) {
+        case IN_CODES: return product1_q8_0_kernel<IN_CODES, OUT_F32>;
+        case IN_F32: return product1_q8_0_kernel<IN_F32, OUT_F32>;
+        case IN_NORM_Q8: return product1_q8_0_kernel<IN_NORM_Q8, OUT_F32>;
+        default: return product1_q8_0_kernel<IN_NORM_F32, OUT_F32>;
+    }
+}
+
+// matvec_q8_0_preq_into for `batch` input vectors, all on the device, with what precedes and follows it in a forward pass
+int flare_launch_product_q8_0(flare_attn_ctx* ctx, const flare_weight* w, const Q8Input& in, int batch, const Q8Output& out) {
+    const int kind = out.oq ? OUT_SILU_Q8 : OUT_F32;
+    if ((in.kind != IN_CODES && !flare_product_quantises(w, batch)) || (kind == OUT_SILU_Q8) != (w->paired != 0) ||
+        (kind == OUT_SILU_Q8 && in.kind != IN_CODES && in.kind != IN_NORM_Q8))
+        return flare_set_error(ctx, FLARE_ERR_STATE, "Q8_0 product: input form %d, output form %d for a matrix of %d x %d", in.kind, kind, w->rows, w->cols);
+    const bool one = batch == 1;
+    ProductParams p;
+    p.w = w->packed; p.in = in; p.out = out;
+    p.rows = w->rows; p.nb = w->cols / 32; p.batch = batch;
+    p.n_units = w->paired ? w->rows / 64 : (w->rows + 15) / 16;
+    p.chunks = (p.nb + CHUNK - 1) / CHUNK;
+    p.cb = (p.nb + p.chunks - 1) / p.chunks;
+    p.stage_bytes = p.cb * BLK;
+    p.n_stages = std::max(2, std::min(MAX_STAGES, 2 * CHUNK * BLK / p.stage_bytes));
+    p.col_groups = (batch + 7) / 8;
+    p.err = ctx->d_err;
+    const int smem = p.n_stages * p.stage_bytes + (one ? 2 * 16 * ROW1 * 4 : p.cb * 512), max_smem = 2 * CHUNK * BLK + CHUNK * 512;
+    ProductKernel kernel = product_kernel(in.kind, kind, one);
     {
         static std::mutex m;
+        static bool done[64][2][2][4] = {};
         std::lock_guard<std::mutex> lock(m);
-        static bool attr_done[64] = {};
-        if (!attr_done[ctx->device & 63]) {
-            FLARE_CUDA_OK(ctx, cudaFuncSetAttribute(matvec_q8_0_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                    WARPS * 32 * TS * (int)sizeof(float)));
-            attr_done[ctx->device & 63] = true;
-        }
+        bool& d = done[ctx->device & 63][one][kind][in.kind];
+        if (!d) FLARE_CUDA_OK(ctx, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem));
+        d = true;
     }
-    p.err = ctx->d_err;
+    // two CTAs fit on an SM; what does not fit at once is walked by those that do
+    const int n_cta = std::min(p.n_units, std::max(1, 2 * ctx->sm_count / p.col_groups));
     ctx->last_launch_overlappable = false;
-    if (w->cols % 256 == 0 && batch == 1 && w->cols <= CHUNK * 32) {
-        const int ring1_smem = WARPS * RING * RING_CHUNK_BYTES + WARPS * GROUP * TS * (int)sizeof(float);
-        {
-            static std::mutex m3;
-            std::lock_guard<std::mutex> lock(m3);
-            static bool ring1_attr[64] = {};
-            if (!ring1_attr[ctx->device & 63]) {
-                FLARE_CUDA_OK(ctx, cudaFuncSetAttribute(matvec_q8_0_ring1_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, ring1_smem));
-                ring1_attr[ctx->device & 63] = true;
-            }
-        }
-        int grid = (w->rows + WARPS - 1) / WARPS;
-        const int max_grid = 148 * 2;                 // two CTAs per SM fit
-        if (grid > max_grid) grid = max_grid;
-        FLARE_CUDA_OK(ctx, flare_launch_pdl(matvec_q8_0_ring1_kernel, dim3(grid), dim3(32 * WARPS), (size_t)ring1_smem, ctx->stream, p));
-        FLARE_LAUNCH_CHECK(ctx);
-        return FLARE_OK;
-    }
-    if (w->cols % 256 == 0 && batch <= 2) {
-        // One or two input vectors: the product is bound by memory, and rows and chunks start on 16-byte boundaries, so
-        // the weights go through a ring of bulk copies.  (From 8 input vectors on the dots dominate and the direct-load
-        // kernel with its many more warps is faster: 212 against 289 us for 128256 x 2048 at batch 8.)
-        const int ring_smem = WARPS * RING * RING_CHUNK_BYTES + smem;
-        {
-            static std::mutex m2;
-            std::lock_guard<std::mutex> lock(m2);
-            static bool ring_attr[64] = {};
-            if (!ring_attr[ctx->device & 63]) {
-                FLARE_CUDA_OK(ctx, cudaFuncSetAttribute(matvec_q8_0_ring_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                        WARPS * RING * RING_CHUNK_BYTES + WARPS * 32 * TS * (int)sizeof(float)));
-                ring_attr[ctx->device & 63] = true;
-            }
-        }
-        // enough CTAs to fill the SMs (3 per SM at batch 1); each warp then walks its rows through the ring
-        int grid = (w->rows + WARPS - 1) / WARPS;
-        const int max_grid = 148 * 3;
-        if (grid > max_grid) grid = max_grid;
-        FLARE_CUDA_OK(ctx, flare_launch_pdl(matvec_q8_0_ring_kernel, dim3(grid), dim3(32 * WARPS), (size_t)ring_smem, ctx->stream, p));
-        FLARE_LAUNCH_CHECK(ctx);
-        return FLARE_OK;
-    }
-    // a row per warp; many more warps than the SMs hold at once are pointless, so large matrices loop
-    int grid = (w->rows + WARPS - 1) / WARPS;
-    const int max_grid = 148 * 8 * 4;
-    if (grid > max_grid) grid = max_grid;
-    FLARE_CUDA_OK(ctx, flare_launch_pdl(matvec_q8_0_kernel, dim3(grid), dim3(32 * WARPS), (size_t)smem, ctx->stream, p));
+    FLARE_CUDA_OK(ctx, flare_launch_pdl(kernel, dim3(n_cta * p.col_groups), dim3(32 * WARPS + (one ? 32 : 0)), (size_t)smem, ctx->stream, p));
     FLARE_LAUNCH_CHECK(ctx);
     return FLARE_OK;
 }
