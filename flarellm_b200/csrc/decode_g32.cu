@@ -51,6 +51,7 @@ struct G32Params {
     int layer_seq0, num_heads, nkv, G, n_split, max_seq;
     int* err;
     uint32_t mask3;         // 0x00030003: a 2-bit code at bit 0 of both 16-bit halves
+    int wait_first;              // the stream may still be writing codes: wait before the first tile request
 };
 
 __device__ __forceinline__ void mma_f16(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
@@ -335,6 +336,7 @@ __global__ void __launch_bounds__(256, 2) decode_g32_kernel(const __grid_constan
         ptx::bulk_load(st + 2 * codes, kmg + (size_t)tile * kmeta_bytes, kmeta_bytes, &full_bar[s]);
         ptx::bulk_load(st + 2 * codes + kmeta_bytes, vmg + (size_t)tile * vmeta_bytes, vmeta_bytes, &full_bar[s]);
     };
+    if (p.wait_first) pdl_wait();
     if (threadIdx.x == 0) {
         for (int s = 0; s < STAGES; s++) { ptx::mbar_init(&full_bar[s], 1); done_cnt[s] = 0; }
         ptx::fence_barrier_init();
@@ -599,8 +601,9 @@ int flare_launch_decode_g32(flare_attn_ctx* ctx, const DecodeArgs& a, const flar
             attr_done[ctx->device & 63] = true;
         }
     }
-    // Programmatic dependent launch as in the Q8_0 path: after one of this library's own attention kernels
-    // (which never write the cache) the next one may start early; both wait before touching q or records.
+    // Programmatic dependent launch as in the Q8_0 path: after a kernel that stores no codes the first tiles are requested
+    // while it drains; the kernel waits before touching q, the ring or records.
+    p.wait_first = ctx->last_launch_overlappable ? 0 : 1;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
@@ -610,7 +613,7 @@ int flare_launch_decode_g32(flare_attn_ctx* ctx, const DecodeArgs& a, const flar
     cfg.dynamicSmemBytes = smem;
     cfg.stream = ctx->stream;
     cfg.attrs = attr;
-    cfg.numAttrs = ctx->last_launch_overlappable ? 1 : 0;
+    cfg.numAttrs = 1;
     bool any_wrapped = false;
     for (int b = 0; b < kv->batch; b++) any_wrapped = any_wrapped || kv->length[b] >= kv->max_seq_len;
     if (any_wrapped) FLARE_CUDA_OK(ctx, cudaLaunchKernelEx(&cfg, decode_g32_kernel<true>, kv->g32_kmap, kv->g32_vmap, p));

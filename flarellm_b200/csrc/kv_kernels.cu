@@ -3,6 +3,7 @@
 // arithmetic operation by operation (IEEE divide, separate multiply and add, round half
 // away from zero) so that codes and scales are byte-identical to the CPU's.
 #include "common.cuh"
+#include <algorithm>
 #include <math_constants.h>
 
 namespace {
@@ -11,48 +12,77 @@ constexpr float kF32Eps = 1.1920929e-07f;
 
 __device__ __forceinline__ int ring_slot(int64_t abs_pos, int max_seq) { return (int)(abs_pos % max_seq); }
 
-// ------------------------------------------------------------------ F32: plain row copy
-__global__ void write_f32_kernel(float* __restrict__ K, float* __restrict__ V, const float* __restrict__ key,
-                                 const float* __restrict__ value, int64_t first_pos, int n_rows, int kv_dim,
-                                 int max_seq) {
-    size_t total = (size_t)n_rows * kv_dim;
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
-        int r = (int)(i / kv_dim), c = (int)(i % kv_dim);
-        // when n_rows > max_seq only the last max_seq rows survive, as with sequential writes
-        if (n_rows - r > max_seq) continue;
-        size_t dst = (size_t)ring_slot(first_pos + r, max_seq) * kv_dim + c;
-        K[dst] = key[i];
-        V[dst] = value[i];
-    }
+// Rows of a prompt go to consecutive ring slots: the host has dropped rows that would be overwritten by later rows of the
+// same call (so n_rows <= max_seq) and reduced the first position to its slot.  A thread moves four values of K and the
+// same four of V, both loads in flight together.
+struct RowSource {
+    const float *key, *value;
+    int first_slot, max_seq;
+    uint32_t units_per_row, n_units;
+};
+__device__ __forceinline__ int row_slot(const RowSource& r, uint32_t row) {
+    const uint32_t s = (uint32_t)r.first_slot + row;
+    return (int)(s >= (uint32_t)r.max_seq ? s - (uint32_t)r.max_seq : s);
+}
+// PACKED: the sources are on 16-byte boundaries
+template <bool PACKED>
+__device__ __forceinline__ float4 load_quad(const float* __restrict__ p, size_t quad) {
+    if (PACKED) return __ldg(reinterpret_cast<const float4*>(p) + quad);
+    const float* q = p + 4 * quad;
+    return make_float4(q[0], q[1], q[2], q[3]);
+}
+
+// T: float4, or float when the sources or the row width do not allow it
+template <typename T>
+__global__ void __launch_bounds__(256) write_f32_kernel(T* __restrict__ K, T* __restrict__ V, const RowSource r) {
+    flare_pdl_wait();
+    flare_pdl_trigger();
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= r.n_units) return;
+    const T k = __ldg(reinterpret_cast<const T*>(r.key) + i), v = __ldg(reinterpret_cast<const T*>(r.value) + i);
+    const uint32_t row = i / r.units_per_row;
+    const size_t dst = (size_t)row_slot(r, row) * r.units_per_row + (i - row * r.units_per_row);
+    K[dst] = k;
+    V[dst] = v;
 }
 
 // ------------------------------------------------------------------ Q8_0
 // flare-core/src/model.rs:5507-5527: amax, d = amax / 127, id = 127 / amax (0 when d == 0),
 // q = round(x * id) as i8 (saturating); the block scale is d rounded to f16 (RNE).
-// One warp per 32-value block, lane = element.
-__global__ void write_q8_kernel(int8_t* __restrict__ Kq, __half* __restrict__ Ks, int8_t* __restrict__ Vq,
-                                __half* __restrict__ Vs, const float* __restrict__ key, const float* __restrict__ value,
-                                int64_t first_pos, int n_rows, int kv_dim, int max_seq) {
-    const int lane = threadIdx.x & 31;
-    const int bpr = kv_dim / 32;
-    const size_t n_blocks = (size_t)n_rows * bpr * 2;   // K blocks then V blocks
-    for (size_t w = (blockIdx.x * (size_t)blockDim.x + threadIdx.x) >> 5; w < n_blocks; w += ((size_t)gridDim.x * blockDim.x) >> 5) {
-        const bool is_v = w >= n_blocks / 2;
-        const size_t bi = is_v ? w - n_blocks / 2 : w;
-        const int r = (int)(bi / bpr), blk = (int)(bi % bpr);
-        if (n_rows - r > max_seq) continue;
-        const float x = (is_v ? value : key)[(size_t)r * kv_dim + blk * 32 + lane];
-        float amax = fabsf(x);
+__device__ __forceinline__ uint32_t q8_code_byte(float x, float id) {
+    const float rr = roundf(__fmul_rn(x, id));
+    const int qi = (rr != rr) ? 0 : (rr >= 127.0f ? 127 : (rr <= -128.0f ? -128 : (int)rr));
+    return (uint32_t)(uint8_t)(int8_t)qi;
+}
+// four values per lane, eight lanes per block: this lane's four codes, and the block's scale on every lane
+__device__ __forceinline__ uint32_t q8_quad(const float4& x, float& d) {
+    float amax = fmaxf(fmaxf(fabsf(x.x), fabsf(x.y)), fmaxf(fabsf(x.z), fabsf(x.w)));
 #pragma unroll
-        for (int off = 16; off; off >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, off));
-        const float d = __fdiv_rn(amax, 127.0f);
-        const float id = (d != 0.0f) ? __fdiv_rn(127.0f, amax) : 0.0f;
-        float rr = roundf(__fmul_rn(x, id));
-        int qi = (rr != rr) ? 0 : (rr >= 127.0f ? 127 : (rr <= -128.0f ? -128 : (int)rr));
-        const int slot = ring_slot(first_pos + r, max_seq);
-        (is_v ? Vq : Kq)[(size_t)slot * kv_dim + blk * 32 + lane] = (int8_t)qi;
-        if (lane == 0) (is_v ? Vs : Ks)[(size_t)slot * bpr + blk] = __float2half_rn(d);
-    }
+    for (int off = 4; off; off >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, off));
+    d = __fdiv_rn(amax, 127.0f);
+    const float id = (d != 0.0f) ? __fdiv_rn(127.0f, amax) : 0.0f;
+    return q8_code_byte(x.x, id) | q8_code_byte(x.y, id) << 8 | q8_code_byte(x.z, id) << 16 | q8_code_byte(x.w, id) << 24;
+}
+// Bound by instruction issue until a lane took four values instead of one (the reduction, the two divisions and the
+// address arithmetic of a block are shared by eight lanes instead of 32) and 64-bit divisions went to the host: 2049 rows of
+// kv_dim 512 and the attention of one query over them, 16 layers, 399 -> 267 us.
+template <bool PACKED>
+__global__ void __launch_bounds__(256) write_q8_kernel(uint32_t* __restrict__ Kq, __half* __restrict__ Ks, uint32_t* __restrict__ Vq,
+                                                       __half* __restrict__ Vs, const RowSource r) {
+    flare_pdl_wait();
+    flare_pdl_trigger();
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    const bool in = i < r.n_units;                    // a block's eight lanes agree: n_units is a multiple of eight
+    const float4 zero = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    const float4 k = in ? load_quad<PACKED>(r.key, i) : zero, v = in ? load_quad<PACKED>(r.value, i) : zero;
+    float kd, vd;
+    const uint32_t kc = q8_quad(k, kd), vc = q8_quad(v, vd);
+    if (!in) return;
+    const uint32_t row = i / r.units_per_row;
+    const size_t dst = (size_t)row_slot(r, row) * r.units_per_row + (i - row * r.units_per_row);
+    Kq[dst] = kc;
+    Vq[dst] = vc;
+    if ((threadIdx.x & 7) == 0) { Ks[dst >> 3] = __float2half_rn(kd); Vs[dst >> 3] = __float2half_rn(vd); }
 }
 
 // ------------------------------------------------------------------ rotary position embedding
@@ -245,15 +275,21 @@ __device__ __forceinline__ float g32_token_value(const __half* ring, const float
     if (tok >= first_pos) return __half2float(__float2half_rn(rows[(size_t)(tok - first_pos) * kv_dim + c]));
     return __half2float(ring[(size_t)(tok % FLARE_G32_RESIDUAL) * kv_dim + c]);
 }
-__global__ void write_g32_groups_kernel(uint8_t* __restrict__ Kq, __half2* __restrict__ Kmeta,
-                                        uint8_t* __restrict__ Vq, __half2* __restrict__ Vmeta,
-                                        const __half* __restrict__ Kres, const __half* __restrict__ Vres,
-                                        const float* __restrict__ key, const float* __restrict__ value,
-                                        int64_t first_pos, int64_t first_trigger, int kv_dim, int max_seq) {
-    // blockIdx.x: trigger index; blockIdx.y: block of 32 channels; 32 warps, warp = w, lane = l
-    const int64_t p = first_trigger + 32 * (int64_t)blockIdx.x;
+// The planes of one layer: bases of sequence 0 and elements between sequences
+struct G32Planes {
+    uint8_t *kq, *vq;
+    __half2 *k_meta, *v_meta;
+    __half *k_res, *v_res;
+    size_t code_stride, k_meta_stride, v_meta_stride, res_stride;
+};
+// The group that trigger p quantises, channels 32 * cblk ..: 32 warps, warp = w, lane = l
+__device__ __forceinline__ void g32_quantise_group(uint8_t* __restrict__ Kq, __half2* __restrict__ Kmeta,
+                                                   uint8_t* __restrict__ Vq, __half2* __restrict__ Vmeta,
+                                                   const __half* Kres, const __half* Vres, const float* __restrict__ key,
+                                                   const float* __restrict__ value, int64_t first_pos, int64_t p, int cblk,
+                                                   int kv_dim, int max_seq) {
     const int64_t tok0 = p - FLARE_G32_RESIDUAL;
-    const int cb = blockIdx.y * 32;
+    const int cb = cblk * 32;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int grp = (int)((tok0 % max_seq) / 32);
     __shared__ uint8_t s_code[32][33];   // [token][channel of this 32-block]
@@ -298,7 +334,40 @@ __global__ void write_g32_groups_kernel(uint8_t* __restrict__ Kq, __half2* __res
         code |= __shfl_xor_sync(0xffffffffu, code, 1);
         code |= __shfl_xor_sync(0xffffffffu, code, 2);
         if ((lane & 3) == 0) Vq[(size_t)slot * (kv_dim / 4) + (cb + lane) / 4] = (uint8_t)code;
-        if (lane == 0) Vmeta[(size_t)slot * (kv_dim / 32) + blockIdx.y] = __halves2half2(__float2half_rn(st.scale), __float2half_rn(st.mn));
+        if (lane == 0) Vmeta[(size_t)slot * (kv_dim / 32) + cblk] = __halves2half2(__float2half_rn(st.scale), __float2half_rn(st.mn));
+    }
+}
+__global__ void write_g32_groups_kernel(uint8_t* __restrict__ Kq, __half2* __restrict__ Kmeta,
+                                        uint8_t* __restrict__ Vq, __half2* __restrict__ Vmeta,
+                                        const __half* __restrict__ Kres, const __half* __restrict__ Vres,
+                                        const float* __restrict__ key, const float* __restrict__ value,
+                                        int64_t first_pos, int64_t first_trigger, int kv_dim, int max_seq) {
+    // blockIdx.x: trigger index; blockIdx.y: block of 32 channels
+    g32_quantise_group(Kq, Kmeta, Vq, Vmeta, Kres, Vres, key, value, first_pos, first_trigger + 32 * (int64_t)blockIdx.x,
+                       blockIdx.y, kv_dim, max_seq);
+}
+// A decode step of the whole batch: blockIdx.y = sequence, blockIdx.x = block of 32 channels, nothing crosses either.  The
+// new row takes the ring place of the first token of the group that it triggers, hence after the quantiser.  (One launch:
+// the launches per sequence that this replaces made a two-layer step of 16 sequences x 32768 take 292 us; it takes 160.)
+__global__ void __launch_bounds__(1024) write_step_g32_kernel(G32Planes c, const float* __restrict__ key, const float* __restrict__ value,
+                                                              const int2* __restrict__ ring, int kv_dim, int max_seq) {
+    flare_pdl_wait();
+    flare_pdl_trigger();
+    const size_t b = blockIdx.y;
+    const int2 r = ring[b];
+    const int64_t p = r.y < max_seq ? r.y : max_seq + r.x;          // congruent to the ring position once it has wrapped
+    __half *Kres = c.k_res + b * c.res_stride, *Vres = c.v_res + b * c.res_stride;
+    key += b * kv_dim; value += b * kv_dim;
+    if (p >= FLARE_G32_RESIDUAL && p % 32 == 0) {      // the host launches full blocks when any sequence is here
+        g32_quantise_group(c.kq + b * c.code_stride, c.k_meta + b * c.k_meta_stride, c.vq + b * c.code_stride,
+                           c.v_meta + b * c.v_meta_stride, Kres, Vres, key, value, p, p, blockIdx.x, kv_dim, max_seq);
+        __syncthreads();
+    }
+    if (threadIdx.x < 32) {
+        const int ch = blockIdx.x * 32 + threadIdx.x;
+        const size_t dst = (size_t)(p % FLARE_G32_RESIDUAL) * kv_dim + ch;
+        Kres[dst] = __float2half_rn(key[ch]);
+        Vres[dst] = __float2half_rn(value[ch]);
     }
 }
 __global__ void write_g32_ring_kernel(__half* __restrict__ Kres, __half* __restrict__ Vres,
@@ -410,18 +479,31 @@ int flare_launch_kv_write(flare_kv* kv, int layer, int seq, int64_t first_pos, i
     const int kvd = kv->kv_dim, ms = kv->max_seq_len;
     switch (kv->dtype) {
         case FLARE_KV_F32:
-            write_f32_kernel<<<grid_for((size_t)n_rows * kvd, 256), 256, 0, st>>>(
-                (float*)kv->plane_ptr(FLARE_PLANE_K, layer, seq), (float*)kv->plane_ptr(FLARE_PLANE_V, layer, seq), d_key,
-                d_value, first_pos, n_rows, kvd, ms);
-            FLARE_LAUNCH_CHECK(ctx);
+        case FLARE_KV_Q8_0: {
+            const int gone = n_rows > ms ? n_rows - ms : 0;        // only the last max_seq rows survive, as with sequential writes
+            const int most = (1 << 30) / kvd;                      // rows of a launch: the kernels count in 32 bits
+            for (int done = gone; done < n_rows; done += most) {
+                RowSource r;
+                r.key = d_key + (size_t)done * kvd; r.value = d_value + (size_t)done * kvd;
+                r.first_slot = (int)((first_pos + done) % ms); r.max_seq = ms;
+                const bool packed = (((uintptr_t)r.key | (uintptr_t)r.value) & 15) == 0;
+                const bool quads = kv->dtype == FLARE_KV_Q8_0 || (packed && kvd % 4 == 0);
+                r.units_per_row = (uint32_t)(quads ? kvd / 4 : kvd);
+                r.n_units = (uint32_t)std::min(most, n_rows - done) * r.units_per_row;
+                const dim3 grid((r.n_units + 255) / 256), block(256);
+                float *k32 = (float*)kv->plane_ptr(FLARE_PLANE_K, layer, seq), *v32 = (float*)kv->plane_ptr(FLARE_PLANE_V, layer, seq);
+                if (kv->dtype == FLARE_KV_F32 && quads)
+                    FLARE_CUDA_OK(ctx, flare_launch_pdl(write_f32_kernel<float4>, grid, block, 0, st, (float4*)k32, (float4*)v32, r));
+                else if (kv->dtype == FLARE_KV_F32)
+                    FLARE_CUDA_OK(ctx, flare_launch_pdl(write_f32_kernel<float>, grid, block, 0, st, k32, v32, r));
+                else
+                    FLARE_CUDA_OK(ctx, flare_launch_pdl(packed ? write_q8_kernel<true> : write_q8_kernel<false>, grid, block, 0, st,
+                        (uint32_t*)kv->plane_ptr(FLARE_PLANE_K_Q, layer, seq), (__half*)kv->plane_ptr(FLARE_PLANE_K_SCALE, layer, seq),
+                        (uint32_t*)kv->plane_ptr(FLARE_PLANE_V_Q, layer, seq), (__half*)kv->plane_ptr(FLARE_PLANE_V_SCALE, layer, seq), r));
+                FLARE_LAUNCH_CHECK(ctx);
+            }
             break;
-        case FLARE_KV_Q8_0:
-            write_q8_kernel<<<grid_for((size_t)n_rows * kvd * 2, 256), 256, 0, st>>>(
-                (int8_t*)kv->plane_ptr(FLARE_PLANE_K_Q, layer, seq), (__half*)kv->plane_ptr(FLARE_PLANE_K_SCALE, layer, seq),
-                (int8_t*)kv->plane_ptr(FLARE_PLANE_V_Q, layer, seq), (__half*)kv->plane_ptr(FLARE_PLANE_V_SCALE, layer, seq),
-                d_key, d_value, first_pos, n_rows, kvd, ms);
-            FLARE_LAUNCH_CHECK(ctx);
-            break;
+        }
         case FLARE_KV_KIVI_REF: {
             write_kivi_ref_codes_kernel<<<n_rows * 2, 128, 0, st>>>(
                 (uint8_t*)kv->plane_ptr(FLARE_PLANE_K_Q, layer, seq), (uint8_t*)kv->plane_ptr(FLARE_PLANE_V_Q, layer, seq),
@@ -488,16 +570,6 @@ int flare_launch_kv_write_step(flare_kv* kv, int layer, const int2* d_ring, cons
             FLARE_LAUNCH_CHECK(ctx);
             return FLARE_OK;
         case FLARE_KV_Q8_0:
-#ifdef FLARE_TUNE
-            if (const char* e = getenv("FLARE_STEP_PDL")) if (!atoi(e)) {
-                write_step_q8_kernel<<<grid_for((size_t)B * kvd * 2, 256), 256, 0, ctx->stream>>>(
-                    (int8_t*)kv->plane_ptr(FLARE_PLANE_K_Q, layer, 0), (__half*)kv->plane_ptr(FLARE_PLANE_K_SCALE, layer, 0),
-                    (int8_t*)kv->plane_ptr(FLARE_PLANE_V_Q, layer, 0), (__half*)kv->plane_ptr(FLARE_PLANE_V_SCALE, layer, 0),
-                    kv->plane_bytes[FLARE_PLANE_K_Q], kv->plane_bytes[FLARE_PLANE_K_SCALE] / 2, d_key, d_value, d_ring, B, kvd, rope);
-                FLARE_LAUNCH_CHECK(ctx);
-                return FLARE_OK;
-            }
-#endif
             FLARE_CUDA_OK(ctx, flare_launch_pdl(write_step_q8_kernel, dim3(grid_for((size_t)B * kvd * 2, 256)), dim3(256), 0, ctx->stream,
                                                 (int8_t*)kv->plane_ptr(FLARE_PLANE_K_Q, layer, 0), (__half*)kv->plane_ptr(FLARE_PLANE_K_SCALE, layer, 0),
                                                 (int8_t*)kv->plane_ptr(FLARE_PLANE_V_Q, layer, 0), (__half*)kv->plane_ptr(FLARE_PLANE_V_SCALE, layer, 0),
@@ -505,8 +577,35 @@ int flare_launch_kv_write_step(flare_kv* kv, int layer, const int2* d_ring, cons
                                                 d_ring, B, kvd, rope));
             FLARE_LAUNCH_CHECK(ctx);
             return FLARE_OK;
+        case FLARE_KV_KIVI_G32: {
+            bool any = false;
+            for (int b = 0; b < B; b++) {
+                const int64_t p = kv->length[b] < kv->max_seq_len ? kv->length[b] : kv->max_seq_len + kv->position[b];
+                any = any || (p >= FLARE_G32_RESIDUAL && p % 32 == 0);
+            }
+            G32Planes c;
+            c.kq = (uint8_t*)kv->plane_ptr(FLARE_PLANE_K_Q, layer, 0); c.vq = (uint8_t*)kv->plane_ptr(FLARE_PLANE_V_Q, layer, 0);
+            c.k_meta = (__half2*)kv->plane_ptr(FLARE_PLANE_K_SCALE, layer, 0); c.v_meta = (__half2*)kv->plane_ptr(FLARE_PLANE_V_SCALE, layer, 0);
+            c.k_res = (__half*)kv->plane_ptr(FLARE_PLANE_K_RES, layer, 0); c.v_res = (__half*)kv->plane_ptr(FLARE_PLANE_V_RES, layer, 0);
+            c.code_stride = kv->plane_bytes[FLARE_PLANE_K_Q];
+            c.k_meta_stride = kv->plane_bytes[FLARE_PLANE_K_SCALE] / sizeof(__half2);
+            c.v_meta_stride = kv->plane_bytes[FLARE_PLANE_V_SCALE] / sizeof(__half2);
+            c.res_stride = kv->plane_bytes[FLARE_PLANE_K_RES] / sizeof(__half);
+            // (grid.y ends at 65535; a larger batch goes in slices)
+            for (int b0 = 0; b0 < B; b0 += 65535) {
+                G32Planes s = c;
+                s.kq += b0 * c.code_stride; s.vq += b0 * c.code_stride; s.k_meta += b0 * c.k_meta_stride; s.v_meta += b0 * c.v_meta_stride;
+                s.k_res += b0 * c.res_stride; s.v_res += b0 * c.res_stride;
+                FLARE_CUDA_OK(ctx, flare_launch_pdl(write_step_g32_kernel, dim3(kvd / 32, std::min(B - b0, 65535)), dim3(any ? 1024 : 32), 0, ctx->stream,
+                                                    s, d_key + (size_t)b0 * kvd, d_value + (size_t)b0 * kvd, d_ring + b0, kvd, kv->max_seq_len));
+                FLARE_LAUNCH_CHECK(ctx);
+            }
+            // without a trigger only f16 ring rows are stored, which no kernel reads before its own wait
+            ctx->last_launch_overlappable = !any && B <= 65535;
+            return FLARE_OK;
+        }
         default:
-            // the 2-bit caches keep per-sequence running state: one sequence at a time (the caller has rotated the rows)
+            // the reference's 2-bit cache keeps running state per sequence: one at a time (the caller has rotated the rows)
             for (int b = 0; b < B; b++) {
                 int64_t abs_pos = kv->length[b] < kv->max_seq_len ? kv->length[b] : kv->max_seq_len + kv->position[b];
                 FLARE_TRY(flare_launch_kv_write(kv, layer, b, abs_pos, kv->length[b], 1, d_key + (size_t)b * kvd,
