@@ -289,44 +289,23 @@ __global__ void __launch_bounds__(32 * WARPS + 32, 2) product1_q8_0_kernel(const
 
     if constexpr (IN != IN_CODES) {                    // one chunk: p.nb <= CHUNK
         float inv_rms = 1.0f;
-        if constexpr (IN != IN_F32) {                  // the sum of squares in the order of the norm kernels
+        if constexpr (IN != IN_F32) {
             if (warp < WARPS) {
-                float e[PER_WARP], sq = 0.0f;
-#pragma unroll
-                for (int k = 0; k < PER_WARP; k++) e[k] = warp + WARPS * k < p.nb ? p.in.x[(warp + WARPS * k) * 32 + lane] : 0.0f;
-#pragma unroll
-                for (int k = 0; k < PER_WARP; k++) sq = fmaf(e[k], e[k], sq);
-#pragma unroll
-                for (int off = 16; off; off >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, off);
+                const float sq = flare_sum_sq_of_warp(p.in.x, p.nb * 32, warp, lane);
                 if (lane == 0) s_sq[warp] = sq;
             }
             __syncthreads();
-            float sum = 0.0f;
-#pragma unroll
-            for (int w = 0; w < WARPS; w++) sum += s_sq[w];
-            inv_rms = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(sum, (float)(p.nb * 32)), p.in.eps)));
+            inv_rms = flare_inv_rms(s_sq, p.nb * 32, p.in.eps);
         }
-        // four values per lane, eight lanes per block
         for (int u = threadIdx.x; u < (p.nb * 8 + 31) / 32 * 32; u += 32 * WARPS + 32) {
             float n[4] = {0.0f, 0.0f, 0.0f, 0.0f};
             if (u < p.nb * 8) {
                 const float4 xv = *reinterpret_cast<const float4*>(p.in.x + 4 * u);
                 n[0] = xv.x; n[1] = xv.y; n[2] = xv.z; n[3] = xv.w;
-                if constexpr (IN != IN_F32) {          // the two norms of the CPU multiply in different order
-                    const float4 nv = __ldg(reinterpret_cast<const float4*>(p.in.norm + 4 * u));
-                    const float nw[4] = {nv.x, nv.y, nv.z, nv.w};
-#pragma unroll
-                    for (int i = 0; i < 4; i++)
-                        n[i] = IN == IN_NORM_Q8 ? __fmul_rn(__fmul_rn(n[i], nw[i]), inv_rms) : __fmul_rn(__fmul_rn(n[i], inv_rms), nw[i]);
-                }
+                if constexpr (IN != IN_F32) flare_norm_quad(n, p.in.norm + 4 * u, inv_rms, IN == IN_NORM_Q8);
             }
-            float amax = fmaxf(fmaxf(fabsf(n[0]), fabsf(n[1])), fmaxf(fabsf(n[2]), fabsf(n[3])));
-#pragma unroll
-            for (int off = 4; off; off >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, off));
-            const float d = __fdiv_rn(amax, 127.0f), id = d != 0.0f ? __fdiv_rn(127.0f, amax) : 0.0f;
-            uint32_t c = 0;
-#pragma unroll
-            for (int i = 0; i < 4; i++) c |= (uint32_t)(uint8_t)flare_to_i8_saturating(roundf(__fmul_rn(n[i], id))) << (8 * i);
+            float d;
+            const uint32_t c = flare_q8_quad(n, d);
             if (u < p.nb * 8) {
                 s_codes[u] = c;
                 if ((u & 7) == 0) s_xs[u >> 3] = d;

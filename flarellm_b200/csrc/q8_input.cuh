@@ -8,18 +8,6 @@ __device__ __forceinline__ int8_t flare_to_i8_saturating(float r) {       // Rus
     return (int8_t)((r != r) ? 0 : (r >= 127.0f ? 127 : (r <= -128.0f ? -128 : (int)r)));
 }
 
-// sum over the block of one value per thread; every thread gets the total (s_red: one float per warp)
-__device__ __forceinline__ float flare_block_sum(float s, float* s_red) {
-#pragma unroll
-    for (int off = 16; off; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
-    __syncthreads();                                  // s_red may still be read from an earlier call
-    if ((threadIdx.x & 31) == 0) s_red[threadIdx.x >> 5] = s;
-    __syncthreads();
-    float t = 0.0f;
-    for (int w = 0; w < (int)(blockDim.x >> 5); w++) t += s_red[w];
-    return t;
-}
-
 // One warp, one block of 32 values (lane = element): amax, scale = amax / 127, code = round(n * (127 / amax)) as i8.
 // Returns this lane's code; every lane gets the scale.
 __device__ __forceinline__ int flare_q8_code(float n, float& scale) {
@@ -36,61 +24,42 @@ __device__ __forceinline__ void flare_quantize_block_of_32(float n, int lane, in
     if (lane == 0) *s_out = scale;
 }
 
-// One input vector of `dim` values quantised by the whole block (any number of warps): plain (norm_weight ==
-// nullptr) or after the RMS norm, n = x * weight * inv_rms.  Up to eight blocks per warp stay in registers between
-// the sum of squares and the quantisation, so that all loads of a pass are in flight together.
-__device__ __forceinline__ void flare_quantize_vector(const float* __restrict__ x, const float* __restrict__ norm_weight,
-                                                      float eps, int dim, int8_t* q_out, float* s_out, float* s_red) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5, nb = dim / 32;
-    if (nb <= 8 * nw) {
-        // the whole vector fits in registers: read once, all loads in flight together
-        float xv[8], wv[8];
+// Four values per lane, eight lanes per block (all of a block's lanes take part): this lane's four codes, and the block's
+// scale on every lane.
+__device__ __forceinline__ uint32_t flare_q8_quad(const float (&n)[4], float& scale) {
+    float amax = fmaxf(fmaxf(fabsf(n[0]), fabsf(n[1])), fmaxf(fabsf(n[2]), fabsf(n[3])));
 #pragma unroll
-        for (int k = 0; k < 8; k++) {
-            const int blk = warp + k * nw;
-            xv[k] = blk < nb ? x[blk * 32 + lane] : 0.0f;
-            wv[k] = (norm_weight && blk < nb) ? norm_weight[blk * 32 + lane] : 1.0f;
-        }
-        float inv_rms = 1.0f;
-        if (norm_weight) {
-            float s = 0.0f;
+    for (int off = 4; off; off >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, off));
+    scale = __fdiv_rn(amax, 127.0f);
+    const float inv_scale = scale != 0.0f ? __fdiv_rn(127.0f, amax) : 0.0f;
+    uint32_t c = 0;
 #pragma unroll
-            for (int k = 0; k < 8; k++) s = fmaf(xv[k], xv[k], s);
-            const float sum_sq = flare_block_sum(s, s_red);
-            inv_rms = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(sum_sq, (float)dim), eps)));
-        }
+    for (int i = 0; i < 4; i++) c |= (uint32_t)(uint8_t)flare_to_i8_saturating(roundf(__fmul_rn(n[i], inv_scale))) << (8 * i);
+    return c;
+}
+
+// The sum of squares of a vector that one warp of eight contributes (warp w: blocks w, w + 8, .., lane = element) and
+// the norm's factor from all eight: one order of additions for every kernel that normalises.
+__device__ __forceinline__ float flare_sum_sq_of_warp(const float* __restrict__ x, int dim, int warp, int lane) {
+    float s = 0.0f;
+#pragma unroll 8
+    for (int i = warp * 32 + lane; i < dim; i += 256) s = fmaf(x[i], x[i], s);
 #pragma unroll
-        for (int k = 0; k < 8; k++) {
-            const int blk = warp + k * nw;
-            if (blk < nb) {
-                const float n = norm_weight ? __fmul_rn(__fmul_rn(xv[k], wv[k]), inv_rms) : xv[k];
-                flare_quantize_block_of_32(n, lane, q_out + blk * 32, s_out + blk);
-            }
-        }
-        return;
-    }
-    float inv_rms = 1.0f;
-    if (norm_weight) {
-        float s = 0.0f;
-        for (int i = threadIdx.x; i < dim; i += blockDim.x) s = fmaf(x[i], x[i], s);
-        const float sum_sq = flare_block_sum(s, s_red);
-        inv_rms = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(sum_sq, (float)dim), eps)));
-    }
-    for (int blk0 = 0; blk0 < nb; blk0 += 8 * nw) {
-        float xv[8], wv[8];
+    for (int off = 16; off; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
+    return s;
+}
+__device__ __forceinline__ float flare_inv_rms(const float* s_sq, int dim, float eps) {
+    float sum = 0.0f;
 #pragma unroll
-        for (int k = 0; k < 8; k++) {
-            const int blk = blk0 + warp + k * nw;
-            xv[k] = blk < nb ? x[blk * 32 + lane] : 0.0f;
-            wv[k] = (norm_weight && blk < nb) ? norm_weight[blk * 32 + lane] : 1.0f;
-        }
+    for (int w = 0; w < 8; w++) sum += s_sq[w];
+    return __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(sum, (float)dim), eps)));
+}
+// The two norms of the CPU multiply in different order: rmsnorm_quantize_q8_0 (x * weight) * inv_rms, rmsnorm_into
+// (x * inv_rms) * weight.
+__device__ __forceinline__ void flare_norm_quad(float (&n)[4], const float* __restrict__ weight, float inv_rms, bool weight_first) {
+    const float4 w4 = __ldg(reinterpret_cast<const float4*>(weight));
+    const float w[4] = {w4.x, w4.y, w4.z, w4.w};
 #pragma unroll
-        for (int k = 0; k < 8; k++) {
-            const int blk = blk0 + warp + k * nw;
-            if (blk < nb) {
-                const float n = norm_weight ? __fmul_rn(__fmul_rn(xv[k], wv[k]), inv_rms) : xv[k];
-                flare_quantize_block_of_32(n, lane, q_out + blk * 32, s_out + blk);
-            }
-        }
-    }
+    for (int i = 0; i < 4; i++)
+        n[i] = weight_first ? __fmul_rn(__fmul_rn(n[i], w[i]), inv_rms) : __fmul_rn(__fmul_rn(n[i], inv_rms), w[i]);
 }
