@@ -12,6 +12,7 @@ from __future__ import annotations
 
 import ctypes as C
 import os
+import threading
 
 import numpy as np
 
@@ -49,6 +50,8 @@ SYMBOLS = [
     ("flare_attn_destroy", _i, [_vp]),
     ("flare_attn_set_stream", _i, [_vp, _vp]),
     ("flare_attn_sync", _i, [_vp]),
+    ("flare_host_alloc", _i, [_vp, _sz, C.POINTER(_vp)]),
+    ("flare_host_free", _i, [_vp]),
     ("flare_attn_last_error", C.c_char_p, [_vp]),
     ("flare_attn_launch_count", C.c_uint64, [_vp]),
     ("flare_attn_backend_name", C.c_char_p, []),
@@ -144,6 +147,89 @@ def _ptr(a):
     return int(a)
 
 
+class _LockedBlock:
+    """Page-locked memory behind one ndarray (its ``base``): back to the pool when the last view of it is gone."""
+
+    def __init__(self, pool, ptr, size, nbytes):
+        self.pool, self.ptr, self.size = pool, ptr, size
+        self.__array_interface__ = {"data": (ptr, False), "shape": (nbytes,), "typestr": "|u1", "version": 3}
+
+    def __del__(self):
+        try:
+            self.pool.put(self.ptr, self.size)
+        except Exception:
+            pass
+
+
+class LockedPool:
+    """Page-locked blocks (powers of two) that large outputs are returned in, so that they cross the bus in one transfer
+    instead of through the driver's staging buffer.  Bounded: beyond ``limit`` bytes, held by arrays or free, an output is an
+    ordinary array.  Shared by all engines of the process; the free blocks go back when the last engine closes."""
+
+    SMALLEST = 128 * 1024      # smaller outputs are page-locked inside the library
+
+    def __init__(self, free, limit=64 << 20):
+        self._free_fn, self.limit = free, limit
+        self._lock = threading.RLock()       # a block may come back from a garbage collection inside take()
+        self._free, self.held, self._users = {}, 0, 0
+
+    def empty(self, alloc, shape, dtype):
+        """An uninitialised array; alloc(bytes) -> pointer or None."""
+        nbytes = int(np.prod(shape, dtype=np.int64)) * np.dtype(dtype).itemsize
+        size = 1 << max(nbytes - 1, 1).bit_length()
+        if nbytes <= self.SMALLEST or size > self.limit:
+            return np.empty(shape, dtype)
+        drop, ptr = [], None
+        with self._lock:
+            if self._free.get(size):
+                ptr = self._free[size].pop()
+            else:
+                for other in sorted(self._free):         # blocks of other sizes make room
+                    while self._free[other] and self.held + size > self.limit:
+                        drop.append(self._free[other].pop())
+                        self.held -= other
+                if self.held + size > self.limit:
+                    size = 0
+                else:
+                    self.held += size
+        for p in drop:
+            self._free_fn(p)
+        if ptr is None and size:
+            ptr = alloc(size)
+            if ptr is None:
+                with self._lock:
+                    self.held -= size
+        if ptr is None:
+            return np.empty(shape, dtype)
+        return np.asarray(_LockedBlock(self, ptr, size, nbytes)).view(dtype).reshape(shape)
+
+    def put(self, ptr, size):
+        with self._lock:
+            if self._users:
+                self._free.setdefault(size, []).append(ptr)
+                return
+            self.held -= size
+        self._free_fn(ptr)
+
+    def add_user(self):
+        with self._lock:
+            self._users += 1
+
+    def drop_user(self):
+        with self._lock:
+            self._users -= 1
+            if self._users:
+                return
+            blocks, self._free = self._free, {}
+            self.held -= sum(size * len(ptrs) for size, ptrs in blocks.items())
+        for ptrs in blocks.values():
+            for p in ptrs:
+                self._free_fn(p)
+
+
+_pool = LockedPool(lambda p: lib().flare_host_free(p))
+
+
 class Engine:
     """One CUDA device + stream (flare_attn_ctx)."""
 
@@ -155,11 +241,13 @@ class Engine:
             raise FlareError(st, "flare_attn_create failed (is a CUDA device present?)")
         self.h = h
         self.device = device
+        _pool.add_user()
 
     def close(self):
         if getattr(self, "h", None):
             self.L.flare_attn_destroy(self.h)
             self.h = None
+            _pool.drop_user()
 
     def __del__(self):
         try:
@@ -211,6 +299,12 @@ class Engine:
     def kv_alloc(self, num_layers, batch, max_seq_len, num_kv_heads, head_dim, dtype=KV_F32) -> "KvCache":
         return KvCache(self, num_layers, batch, max_seq_len, num_kv_heads, head_dim, dtype)
 
+    def _empty(self, shape, dtype=np.float32) -> np.ndarray:
+        def alloc(n):
+            p = _vp()
+            return p.value if self.L.flare_host_alloc(self.h, n, C.byref(p)) == OK else None
+        return _pool.empty(alloc, shape, dtype)
+
     # ---- attention -------------------------------------------------------------------------
     def decode(self, kv: "KvCache", layer, num_heads, q, n_q=1, attend_len=None, softcap=0.0, out=None):
         """q: host ndarray [batch][n_q][num_heads][head_dim] f32, or a device pointer (int) with
@@ -220,7 +314,7 @@ class Engine:
             q = np.ascontiguousarray(q, dtype=np.float32)
             assert q.size == kv.batch * n_q * num_heads * kv.head_dim
             if out is None:
-                out = np.empty((kv.batch, n_q, num_heads, kv.head_dim), dtype=np.float32)
+                out = self._empty((kv.batch, n_q, num_heads, kv.head_dim))
         al = None
         if attend_len is not None:
             al_arr = np.ascontiguousarray(attend_len, dtype=np.int32)
@@ -245,7 +339,7 @@ class Engine:
             key, value, q = (a if (a.dtype == np.float32 and a.flags["C_CONTIGUOUS"]) else
                              np.ascontiguousarray(a, dtype=np.float32) for a in (key, value, q))
             if out is None:
-                out = np.empty((kv.batch, 1, num_heads, kv.head_dim), dtype=np.float32)
+                out = self._empty((kv.batch, 1, num_heads, kv.head_dim))
         self.check(self.L.flare_decode_step(self.h, kv.h, layer, num_heads, _ptr(key), _ptr(value), _ptr(q), _ptr(out),
                                             int(on_device)))
         return out
@@ -300,7 +394,7 @@ class Engine:
             x = np.ascontiguousarray(x, dtype=np.float32).reshape(-1, w.cols)
             batch = x.shape[0]
             if out is None:
-                out = np.empty((batch, w.rows), dtype=np.float32)
+                out = self._empty((batch, w.rows))
             out_ptr = _ptr(out)
         self.check(self.L.flare_matvec_q8_0(self.h, w.h, _ptr(x), batch, out_ptr, int(on_device)))
         return out
@@ -367,8 +461,7 @@ class Engine:
             want = np.float32 if in_dtype == DT_F32 else np.uint16
             q, k, v = (np.ascontiguousarray(a, dtype=want) for a in (q, k, v))
             if out is None:
-                out = np.empty((batch, seq_len, num_heads, head_dim),
-                               dtype=np.float32 if out_dtype == DT_F32 else np.uint16)
+                out = self._empty((batch, seq_len, num_heads, head_dim), np.float32 if out_dtype == DT_F32 else np.uint16)
         self.check(self.L.flare_prefill_attn(self.h, _ptr(q), _ptr(k), _ptr(v), in_dtype, batch, seq_len, num_heads,
                                              num_kv_heads, head_dim, window, softcap, _ptr(out), out_dtype,
                                              int(on_device)))
@@ -453,7 +546,7 @@ class ResidentModel:
         x = np.ascontiguousarray(token_embed, dtype=np.float32).reshape(-1, self.cfg.hidden_dim)
         pos = np.ascontiguousarray(positions, dtype=np.int64).reshape(-1)
         assert x.shape[0] == kv.batch == pos.size
-        logits = np.empty((kv.batch, self.cfg.vocab_size), dtype=np.float32)
+        logits = self.eng._empty((kv.batch, self.cfg.vocab_size))
         self.eng.check(self.L.flare_forward_token(self.eng.h, self.h, kv.h, _ptr(x), _ptr(pos), _ptr(logits)))
         return logits
 

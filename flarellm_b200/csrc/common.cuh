@@ -42,6 +42,8 @@ struct flare_attn_ctx {
     void* h_pinned = nullptr;    size_t pinned_bytes = 0;
     // ring of page-locked staging slots for small host inputs (new K/V rows): the caller's buffer is
     // copied here by the CPU, the transfer to the device is then asynchronous and the call need not wait
+    void* h_out = nullptr;       // page-locked, device-mapped: small outputs on their way to pageable memory
+    void* d_out = nullptr;       // the device's address of the same
     void* h_rows = nullptr;      size_t rows_slot_bytes = 0;
     cudaEvent_t rows_events[FLARE_ROW_SLOTS] = {};
     uint64_t rows_counter = 0;
