@@ -27,13 +27,25 @@ __global__ void bf16_to_f32_kernel(const __nv_bfloat16* __restrict__ in, float* 
 // f32 -> f16 for the tensor cores.  f16 keeps 11 significant bits (bf16: 8) but spans only 6e-5 .. 65504 at
 // full precision, so each tensor is first scaled by a power of two (exact) that puts its largest magnitude in
 // [2^14, 2^15); the attention kernel undoes the scaling in its softmax scale and its final normalisation.
-__global__ void amax3_kernel(const float* __restrict__ q, size_t qn, const float* __restrict__ k,
-                             const float* __restrict__ v, size_t kn, unsigned* __restrict__ amax_bits) {
+// Both passes are bound by HBM; V: float4 (counts are multiples of the head size), or float where a pointer given by the
+// caller is not on a 16-byte boundary.
+__device__ __forceinline__ float amax_of(float x) { return fabsf(x); }
+__device__ __forceinline__ float amax_of(const float4& x) { return fmaxf(fmaxf(fabsf(x.x), fabsf(x.y)), fmaxf(fabsf(x.z), fabsf(x.w))); }
+__device__ __forceinline__ void store_half(__half* out, size_t i, float x, float scale) { out[i] = __float2half_rn(x * scale); }
+__device__ __forceinline__ void store_half(__half* out, size_t i, const float4& x, float scale) {
+    const __half2 lo = __floats2half2_rn(x.x * scale, x.y * scale), hi = __floats2half2_rn(x.z * scale, x.w * scale);
+    reinterpret_cast<uint2*>(out)[i] = make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
+}
+template <typename V>
+__global__ void __launch_bounds__(256) amax3_kernel(const V* __restrict__ q, size_t qn, const V* __restrict__ k,
+                                                    const V* __restrict__ v, size_t kn, unsigned* __restrict__ amax_bits) {
     __shared__ unsigned s_red[3][8];
     float m[3] = {0.0f, 0.0f, 0.0f};
     const size_t stride = (size_t)gridDim.x * blockDim.x, i0 = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
-    for (size_t i = i0; i < qn; i += stride) m[0] = fmaxf(m[0], fabsf(q[i]));
-    for (size_t i = i0; i < kn; i += stride) { m[1] = fmaxf(m[1], fabsf(k[i])); m[2] = fmaxf(m[2], fabsf(v[i])); }
+    #pragma unroll 4
+    for (size_t i = i0; i < qn; i += stride) m[0] = fmaxf(m[0], amax_of(q[i]));
+#pragma unroll 2
+    for (size_t i = i0; i < kn; i += stride) { m[1] = fmaxf(m[1], amax_of(k[i])); m[2] = fmaxf(m[2], amax_of(v[i])); }
 #pragma unroll
     for (int t = 0; t < 3; t++) {
 #pragma unroll
@@ -54,15 +66,18 @@ __device__ __forceinline__ float f16_fit_scale(unsigned amax_bits) {
     frexpf(a, &e);                                          // a = m 2^e, m in [0.5, 1)
     return ldexpf(1.0f, max(-40, min(40, 15 - e)));         // a * scale in [2^14, 2^15) unless a is extreme
 }
-__global__ void f32_to_f16_scaled_kernel(const float* __restrict__ q, size_t qn, const float* __restrict__ k,
-                                         const float* __restrict__ v, size_t kn, __half* __restrict__ wq,
-                                         __half* __restrict__ wk, __half* __restrict__ wv,
-                                         const unsigned* __restrict__ amax_bits, float* __restrict__ descale) {
+template <typename V>
+__global__ void __launch_bounds__(256) f32_to_f16_scaled_kernel(const V* __restrict__ q, size_t qn, const V* __restrict__ k,
+                                                                const V* __restrict__ v, size_t kn, __half* __restrict__ wq,
+                                                                __half* __restrict__ wk, __half* __restrict__ wv,
+                                                                const unsigned* __restrict__ amax_bits, float* __restrict__ descale) {
     const float sq = f16_fit_scale(amax_bits[0]), sk = f16_fit_scale(amax_bits[1]), sv = f16_fit_scale(amax_bits[2]);
     if (blockIdx.x == 0 && threadIdx.x == 0) { descale[0] = 1.0f / (sq * sk); descale[1] = 1.0f / sv; }
     const size_t stride = (size_t)gridDim.x * blockDim.x, i0 = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
-    for (size_t i = i0; i < qn; i += stride) wq[i] = __float2half_rn(q[i] * sq);
-    for (size_t i = i0; i < kn; i += stride) { wk[i] = __float2half_rn(k[i] * sk); wv[i] = __float2half_rn(v[i] * sv); }
+#pragma unroll 4
+    for (size_t i = i0; i < qn; i += stride) store_half(wq, i, q[i], sq);
+#pragma unroll 2
+    for (size_t i = i0; i < kn; i += stride) { store_half(wk, i, k[i], sk); store_half(wv, i, v[i], sv); }
 }
 
 int make_qkv_map(CUtensorMap* m, const void* base, int hd, int heads, int S, int batch, bool f16) {
@@ -143,11 +158,18 @@ int flare_launch_prefill(flare_attn_ctx* ctx, const PrefillArgs& a) {
         unsigned* amax = (unsigned*)((char*)ctx->d_conv + halves);
         float* descale = (float*)(amax + 4);
         FLARE_CUDA_OK(ctx, cudaMemsetAsync(amax, 0, 16, ctx->stream));
-        amax3_kernel<<<conv_grid, conv_threads, 0, ctx->stream>>>((const float*)a.q, qn, (const float*)a.k, (const float*)a.v, kn, amax);
-        FLARE_LAUNCH_CHECK(ctx);
-        f32_to_f16_scaled_kernel<<<conv_grid, conv_threads, 0, ctx->stream>>>((const float*)a.q, qn, (const float*)a.k,
-                                                                              (const float*)a.v, kn, w, w + qn, w + qn + kn,
-                                                                              amax, descale);
+        const bool quads = (((uintptr_t)a.q | (uintptr_t)a.k | (uintptr_t)a.v) & 15) == 0;
+        if (quads) {
+            const float4 *q4 = (const float4*)a.q, *k4 = (const float4*)a.k, *v4 = (const float4*)a.v;
+            amax3_kernel<float4><<<conv_grid, conv_threads, 0, ctx->stream>>>(q4, qn / 4, k4, v4, kn / 4, amax);
+            FLARE_LAUNCH_CHECK(ctx);
+            f32_to_f16_scaled_kernel<float4><<<conv_grid, conv_threads, 0, ctx->stream>>>(q4, qn / 4, k4, v4, kn / 4, w, w + qn, w + qn + kn, amax, descale);
+        } else {
+            const float *q1 = (const float*)a.q, *k1 = (const float*)a.k, *v1 = (const float*)a.v;
+            amax3_kernel<float><<<conv_grid, conv_threads, 0, ctx->stream>>>(q1, qn, k1, v1, kn, amax);
+            FLARE_LAUNCH_CHECK(ctx);
+            f32_to_f16_scaled_kernel<float><<<conv_grid, conv_threads, 0, ctx->stream>>>(q1, qn, k1, v1, kn, w, w + qn, w + qn + kn, amax, descale);
+        }
         FLARE_LAUNCH_CHECK(ctx);
         q = w; k = w + qn; v = w + qn + kn;
         a2.f16_ops = 1; a2.descale = descale;
