@@ -148,7 +148,7 @@ def _ptr(a):
 
 
 class _LockedBlock:
-    """Page-locked memory behind one ndarray (its ``base``): back to the pool when the last view of it is gone."""
+    """Page-locked memory behind one ndarray: back to the pool when the last view of it is gone."""
 
     def __init__(self, pool, ptr, size, nbytes):
         self.pool, self.ptr, self.size = pool, ptr, size
@@ -162,45 +162,42 @@ class _LockedBlock:
 
 
 class LockedPool:
-    """Page-locked blocks (powers of two) that large outputs are returned in, so that they cross the bus in one transfer
-    instead of through the driver's staging buffer.  Bounded: beyond ``limit`` bytes, held by arrays or free, an output is an
-    ordinary array.  Shared by all engines of the process; the free blocks go back when the last engine closes."""
+    """Page-locked blocks that large outputs are returned in, so that they cross the bus in one transfer instead of through
+    the driver's staging buffer.  Locking pages costs milliseconds, a transfer saves a few hundred microseconds: a size gets
+    a block of its own only when it is asked for again, a free block up to twice too large is as good, and blocks are not
+    exchanged for others.  Bounded: beyond ``limit`` bytes, held by arrays or free, an output is an ordinary array.
+    Shared by all engines of the process; the free blocks go back when the last engine closes."""
 
     SMALLEST = 128 * 1024      # smaller outputs are page-locked inside the library
 
     def __init__(self, free, limit=64 << 20):
         self._free_fn, self.limit = free, limit
-        self._lock = threading.RLock()       # a block may come back from a garbage collection inside take()
-        self._free, self.held, self._users = {}, 0, 0
+        self._lock = threading.RLock()       # a block may come back from a garbage collection inside empty()
+        self._free, self._seen, self.held, self._users = {}, set(), 0, 0
 
     def empty(self, alloc, shape, dtype):
         """An uninitialised array; alloc(bytes) -> pointer or None."""
         nbytes = int(np.prod(shape, dtype=np.int64)) * np.dtype(dtype).itemsize
-        size = 1 << max(nbytes - 1, 1).bit_length()
-        if nbytes <= self.SMALLEST or size > self.limit:
+        if nbytes <= self.SMALLEST or nbytes > self.limit:
             return np.empty(shape, dtype)
-        drop, ptr = [], None
+        step = 1 << max(nbytes.bit_length() - 4, 12)      # sizes in steps of an eighth or less
+        size, ptr = (nbytes + step - 1) // step * step, None
         with self._lock:
-            if self._free.get(size):
+            fits = [n for n, blocks in self._free.items() if blocks and size <= n <= 2 * size]
+            if fits:
+                size = min(fits)
                 ptr = self._free[size].pop()
+            elif size in self._seen and self.held + size <= self.limit:
+                self.held += size
             else:
-                for other in sorted(self._free):         # blocks of other sizes make room
-                    while self._free[other] and self.held + size > self.limit:
-                        drop.append(self._free[other].pop())
-                        self.held -= other
-                if self.held + size > self.limit:
-                    size = 0
-                else:
-                    self.held += size
-        for p in drop:
-            self._free_fn(p)
-        if ptr is None and size:
+                self._seen.add(size)
+                return np.empty(shape, dtype)
+        if ptr is None:
             ptr = alloc(size)
             if ptr is None:
                 with self._lock:
                     self.held -= size
-        if ptr is None:
-            return np.empty(shape, dtype)
+                return np.empty(shape, dtype)
         return np.asarray(_LockedBlock(self, ptr, size, nbytes)).view(dtype).reshape(shape)
 
     def put(self, ptr, size):
@@ -220,7 +217,7 @@ class LockedPool:
             self._users -= 1
             if self._users:
                 return
-            blocks, self._free = self._free, {}
+            blocks, self._free, self._seen = self._free, {}, set()
             self.held -= sum(size * len(ptrs) for size, ptrs in blocks.items())
         for ptrs in blocks.values():
             for p in ptrs:
